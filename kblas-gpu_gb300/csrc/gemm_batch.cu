@@ -19,8 +19,11 @@
 // a matrix with m <= 0 or n <= 0 is skipped.
 #include <stdio.h>
 
+#include <type_traits>
+
 #include <cuComplex.h>
 
+#include "gemm_split.cuh"
 #include "gemm_tile.cuh"
 #include "kblas_internal.h"
 #include "launch_util.h"
@@ -64,8 +67,23 @@ static inline bool trans_flag(char c, int &t) {
 
 template <typename T, class AccA, class AccB, class AccC, class Dims>
 static int launch_gemm(KBlasHandle *h, int ta, int tb, T alpha, AccA A, AccB B, T beta, AccC Cm,
-                       Dims dims, long long batch, long long tiles_hint) {
+                       Dims dims, long long batch, long long tiles_hint, int mmax, int nmax,
+                       int kmax) {
   if (batch > 0x7fffffffLL) return KBLAS_NotSupported;
+  if constexpr (std::is_same<T, double>::value) {
+    if (alpha != 0.0 && sp_worthwhile(mmax, nmax, kmax)) {
+      dim3 grid;
+      int ncp;
+      sp_grid(h, batch, mmax, nmax, grid, ncp);
+      auto kern = gemm_split_kernel<false, AccA, AccB, AccC, Dims>;
+      int st = set_smem(kern, SP_SMEM);
+      if (st != KBLAS_Success) return st;
+      kern<<<grid, SP_NT, SP_SMEM, h->stream>>>(ta, tb, TILE_FULL, alpha, A, B, beta, Cm, dims, ncp,
+                                                h->d_status);
+      KGB_LAUNCH_CHECK("gemm_split_kernel");
+      return KBLAS_Success;
+    }
+  }
   dim3 grid((unsigned)batch, tile_slots(h, batch, tiles_hint));
   gemm_batch_kernel<T><<<grid, GT_NT, 0, h->stream>>>(ta, tb, alpha, A, B, beta, Cm, dims, batch);
   KGB_LAUNCH_CHECK("gemm_batch_kernel");
@@ -98,7 +116,7 @@ static int gemm_strided(KBlasHandle *h, char transA, char transB, int m, int n, 
   DimsU<6> dims{{m, n, k, lda, ldb, ldc}};
   return launch_gemm<T>(h, ta, tb, alpha, Strided<T>{const_cast<T *>(A), sA},
                         Strided<T>{const_cast<T *>(B), sB}, beta, Strided<T>{C, sC}, dims, batch,
-                        ceil_div(m, GT) * ceil_div(n, GT));
+                        ceil_div(m, GT) * ceil_div(n, GT), m, n, k);
 }
 
 template <typename T>
@@ -113,7 +131,7 @@ static int gemm_array(KBlasHandle *h, char transA, char transB, int m, int n, in
   DimsU<6> dims{{m, n, k, lda, ldb, ldc}};
   return launch_gemm<T>(h, ta, tb, alpha, PtrArr<T>{const_cast<T **>(A)},
                         PtrArr<T>{const_cast<T **>(B)}, beta, PtrArr<T>{C}, dims, batch,
-                        ceil_div(m, GT) * ceil_div(n, GT));
+                        ceil_div(m, GT) * ceil_div(n, GT), m, n, k);
 }
 
 template <typename T>
@@ -121,7 +139,6 @@ static int gemm_vbatch(KBlasHandle *h, char transA, char transB, const int *m, c
                        const int *k, int max_m, int max_n, int max_k, T alpha, const T **A,
                        const int *lda, const T **B, const int *ldb, T beta, T **C, const int *ldc,
                        int batch) {
-  (void)max_k;
   if (!h) return KBLAS_Error_NotInitialized;
   int ta, tb;
   if (batch < 1 || !trans_flag(transA, ta) || !trans_flag(transB, tb)) return KBLAS_Error_WrongInput;
@@ -129,7 +146,7 @@ static int gemm_vbatch(KBlasHandle *h, char transA, char transB, const int *m, c
   const long long hint = (max_m > 0 && max_n > 0) ? ceil_div(max_m, GT) * ceil_div(max_n, GT) : 0;
   DimsV<6> dims{{m, n, k, lda, ldb, ldc}};
   return launch_gemm<T>(h, ta, tb, alpha, PtrArr<T>{const_cast<T **>(A)},
-                        PtrArr<T>{const_cast<T **>(B)}, beta, PtrArr<T>{C}, dims, batch, hint);
+                        PtrArr<T>{const_cast<T **>(B)}, beta, PtrArr<T>{C}, dims, batch, hint, max_m, max_n, max_k);
 }
 
 template <typename T>

@@ -11,9 +11,12 @@
 // time, and a 2 x 2 register tile of C per thread.
 #include <stdio.h>
 
+#include <type_traits>
+
 #include <cuComplex.h>
 
 #include "device_util.cuh"
+#include "gemm_split.cuh"
 #include "gemm_tile.cuh"
 #include "kblas_internal.h"
 #include "launch_util.h"
@@ -109,6 +112,30 @@ static int launch_syrk(KBlasHandle *h, int m, int k, bool trans, T alpha, AccA A
   return KBLAS_Success;
 }
 
+// Double precision from sp_worthwhile sizes on: the tensor-core kernel of
+// gemm_split.cuh, either triangle.
+template <typename T, class AccA, class AccC>
+static int launch_syrk_any(KBlasHandle *h, bool upper, int m, int k, bool trans, T alpha, AccA A,
+                           int lda, T beta, AccC Cm, int ldc, long long batch) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (alpha != 0.0 && batch <= 0x7fffffffLL && sp_worthwhile(m, m, k)) {
+      dim3 grid;
+      int ncp;
+      sp_grid(h, batch, m, m, grid, ncp);
+      auto kern = gemm_split_kernel<true, AccA, AccA, AccC, DimsU<4>>;
+      int st = set_smem(kern, SP_SMEM);
+      if (st != KBLAS_Success) return st;
+      kern<<<grid, SP_NT, SP_SMEM, h->stream>>>(trans ? 1 : 0, trans ? 0 : 1,
+                                                upper ? TILE_UPPER : TILE_LOWER, alpha, A, A, beta,
+                                                Cm, DimsU<4>{{m, k, lda, ldc}}, ncp, h->d_status);
+      KGB_LAUNCH_CHECK("gemm_split_kernel");
+      return KBLAS_Success;
+    }
+  }
+  if (upper) return launch_syrk_upper<T>(h, m, k, trans, alpha, A, lda, beta, Cm, ldc, batch);
+  return launch_syrk<T>(h, m, k, trans, alpha, A, lda, beta, Cm, ldc, batch);
+}
+
 static inline int check_syrk(KBlasHandle *h, char uplo, char trans, int m, int n, int lda, int ldb,
                              int batch) {
   if (!h) return KBLAS_Error_NotInitialized;
@@ -127,11 +154,9 @@ static int syrk_strided(KBlasHandle *h, char uplo, char trans, int m, int n, T a
   if (st != KBLAS_Success) return st;
   if (m == 0 || batch == 0) return KBLAS_Success;
   if (!B || (n > 0 && !A) || (batch > 1 && sB < (long long)ldb * m)) return KBLAS_Error_WrongInput;
-  if (is_upper(uplo))
-    return launch_syrk_upper<T>(h, m, n, is_trans(trans), alpha, Strided<T>{const_cast<T *>(A), sA},
-                                lda, beta, Strided<T>{B, sB}, ldb, batch);
-  return launch_syrk<T>(h, m, n, is_trans(trans), alpha, Strided<T>{const_cast<T *>(A), sA}, lda,
-                        beta, Strided<T>{B, sB}, ldb, batch);
+  return launch_syrk_any<T>(h, is_upper(uplo), m, n, is_trans(trans), alpha,
+                            Strided<T>{const_cast<T *>(A), sA}, lda, beta, Strided<T>{B, sB}, ldb,
+                            batch);
 }
 
 template <typename T>
@@ -141,11 +166,8 @@ static int syrk_array(KBlasHandle *h, char uplo, char trans, int m, int n, T alp
   if (st != KBLAS_Success) return st;
   if (m == 0 || batch == 0) return KBLAS_Success;
   if (!B || (n > 0 && !A)) return KBLAS_Error_WrongInput;
-  if (is_upper(uplo))
-    return launch_syrk_upper<T>(h, m, n, is_trans(trans), alpha, PtrArr<T>{const_cast<T **>(A)}, lda,
-                                beta, PtrArr<T>{B}, ldb, batch);
-  return launch_syrk<T>(h, m, n, is_trans(trans), alpha, PtrArr<T>{const_cast<T **>(A)}, lda, beta,
-                        PtrArr<T>{B}, ldb, batch);
+  return launch_syrk_any<T>(h, is_upper(uplo), m, n, is_trans(trans), alpha,
+                            PtrArr<T>{const_cast<T **>(A)}, lda, beta, PtrArr<T>{B}, ldb, batch);
 }
 
 }  // namespace kgb
