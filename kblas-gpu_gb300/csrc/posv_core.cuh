@@ -39,6 +39,7 @@
 namespace kgb {
 
 constexpr int PC_NT = 256;     // threads per persistent CTA
+constexpr int PC_MAX_N = 1024; // largest order the panel path takes
 constexpr int PC_NCLS = 8;     // size classes (KBLAS_POSV_TUNING_CLASSES)
 constexpr int PC_MR = 4;       // right-hand sides per residual sweep (panel path)
 // The mixed panel path runs its trailing updates on the tensor cores when a
@@ -140,7 +141,7 @@ struct SysArgs {
 };
 
 struct ItemArgs {
-  int uniform;          // 1: item q = systems [q*spi, (q+1)*spi)
+  int uniform;          // 1: item q = systems [q*spi, (q+1)*spi); 2: of perm[0 .. *nitems_p)
   long long batch;
   int n_uniform;
   const int4 *items;    // (n, start, count, -) into perm
@@ -671,7 +672,7 @@ __device__ __forceinline__ void prefetch_item(const SysArgs &sys, const ItemArgs
   const int pairs = count * n;  // (system, column) pairs
   for (int pc = threadIdx.x; pc < pairs; pc += blockDim.x) {
     const int k = pc / n, j = pc - k * n;
-    const long long sidx = it.uniform ? (long long)start + k : (long long)it.perm[start + k];
+    const long long sidx = it.uniform == 1 ? (long long)start + k : (long long)it.perm[start + k];
     int m, lda, ldb;
     double *A, *B;
     sys.get(sidx, m, A, lda, B, ldb);
@@ -719,6 +720,7 @@ posv_persistent_kernel(SysArgs sys, ItemArgs it, OutArgs out, PosvCfg cfg, int s
   TcCtx tcx{use_tc ? s_tmem : 0u, &s_tcbar, nullptr, &s_abort, out.status, 0u};
   long long first = 0, nitems;
   if (it.uniform) {
+    if (it.uniform == 2) it.batch = *it.nitems_p;
     const int spi = cfg.spi[pc_class(cfg, it.n_uniform)];
     nitems = (it.batch + spi - 1) / spi;
   } else {
@@ -754,7 +756,7 @@ posv_persistent_kernel(SysArgs sys, ItemArgs it, OutArgs out, PosvCfg cfg, int s
     int m = 0, lda = 1, ldb = 1;
     double *A = nullptr, *B = nullptr;
     if (active) {
-      sidx = it.uniform ? (long long)start + team_id : (long long)it.perm[start + team_id];
+      sidx = it.uniform == 1 ? (long long)start + team_id : (long long)it.perm[start + team_id];
       sys.get(sidx, m, A, lda, B, ldb);
     }
     unsigned char *base = smem + (size_t)team_id * tb;

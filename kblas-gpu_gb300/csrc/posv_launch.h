@@ -8,11 +8,12 @@
 #include "kblas_internal.h"
 #include "launch_util.h"
 #include "posv_core.cuh"
+#include "posv_fix.h"
 #include "tuning_table.h"
 
 namespace kgb {
 
-constexpr int PC_MAX_N = 1024;          // largest order the persistent kernels take
+
 constexpr size_t PC_SMEM_BUDGET = 220 * 1024;
 
 struct PosvPlan {
@@ -177,13 +178,16 @@ struct PosvWs {
   size_t off = 0;      // int[max_n + 1]   first slot of order n in perm
   size_t ioff = 0;     // int[max_n + 1]   first item of order n
   size_t cursor = 0;   // int[max_n + 1]
+  size_t redo = 0;     // int[batch]        plain FP64: systems for the FP64 path
   size_t perm = 0;     // int[batch]
   size_t items = 0;    // int4[batch]
   size_t scratch = 0;  // grid * slot_bytes
   size_t total = 0;
 };
 
-static inline PosvWs posv_ws_layout(int max_n, long long batch, bool binned, const PosvPlan &pl) {
+// fix: the plain FP64 routines, whose systems run in fixed point first.
+static inline PosvWs posv_ws_layout(KBlasHandle *h, int max_n, long long batch, bool binned,
+                                    bool fix, const PosvPlan &pl) {
   PosvWs w;
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -198,10 +202,16 @@ static inline PosvWs posv_ws_layout(int max_n, long long batch, bool binned, con
     w.off = take(nb);
     w.ioff = take(nb);
     w.cursor = take(nb);
+  }
+  if (fix) w.redo = take((size_t)batch * sizeof(int));
+  if (binned) {
     w.perm = take((size_t)batch * sizeof(int));
     w.items = take((size_t)batch * sizeof(int4));
   }
-  w.scratch = take((size_t)pl.grid * pl.slot_bytes);
+  // (used by one launch after the other)
+  size_t scr = (size_t)pl.grid * pl.slot_bytes;
+  const size_t fscr = fix ? fix_scratch_bytes(h, max_n) : 0;
+  w.scratch = take(scr > fscr ? scr : fscr);
   w.total = o;
   return w;
 }

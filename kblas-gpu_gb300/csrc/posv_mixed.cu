@@ -24,7 +24,7 @@ size_t mixed_posv_ws_bytes(KBlasHandle *h, int n, long long batch) {
   PosvPlan pl;
   const int st = n > 32 ? plan_posv<true, 2>(h, n, pl) : plan_posv<true, 1>(h, n, pl);
   if (st != KBLAS_Success) return 0;
-  return posv_ws_layout(n, batch, false, pl).total;
+  return posv_ws_layout(h, n, batch, false, false, pl).total;
 }
 
 static int mixed_uniform(KBlasHandle *h, char side, char uplo, int m, int n, SysArgs sys, int batch,
@@ -47,7 +47,7 @@ static int mixed_uniform(KBlasHandle *h, char side, char uplo, int m, int n, Sys
   PosvPlan pl;
   int st = n > 32 ? plan_posv<true, 2>(h, n, pl) : plan_posv<true, 1>(h, n, pl);
   if (st != KBLAS_Success) return st;
-  const PosvWs ws = posv_ws_layout(n, batch, false, pl);
+  const PosvWs ws = posv_ws_layout(h, n, batch, false, false, pl);
   if (ws.total > h->ws.allocated.d_data_bytes || !h->ws.d_data) return KBLAS_InsufficientWorkspace;
   char *base = static_cast<char *>(h->ws.d_data);
   int *header = reinterpret_cast<int *>(base + ws.header);

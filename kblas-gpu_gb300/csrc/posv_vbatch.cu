@@ -16,6 +16,8 @@
 //                          systems of equal n, sized by the tuning table)
 //   4. vb_scatter       -- counting-sort the system indices into the slices
 //   5. posv_persistent_kernel -- CTAs pull items from the queue
+// Plain FP64, orders above 32: fix_posv_kernel (posv_fix.cu, one launch per class
+// of orders) takes 5's place, and what it marks goes through 2 to 5 once more.
 // Largest-first ordering keeps the tail of the persistent launch short (the
 // cost per system spans n^3 over a 32x range of n).
 #include <stdio.h>
@@ -26,10 +28,12 @@
 namespace kgb {
 
 __global__ void vb_count(long long batch, const int *n, const int *m, const int *lda,
-                         const int *ldb, int max_m, int max_n, int *cnt, int *info, int *iter)
+                         const int *ldb, int max_m, int max_n, int *cnt, int *info, int *iter,
+                         const int *only)
 {
   for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < batch;
        b += (long long)gridDim.x * blockDim.x) {
+    if (only && !only[b]) continue;
     const int nn = n[b], mm = m[b], la = lda[b], lb = ldb[b];
     int bad = 0;
     // argument positions of kblasDposv_vbatch: 4 m, 5 n, 6 max_m, 7 max_n, 9 lda, 11 ldb
@@ -79,10 +83,11 @@ __global__ void vb_plan(int max_n, const int *cnt, int *off, int *ioff, int4 *it
 
 __global__ void vb_scatter(long long batch, const int *n, const int *m, const int *lda,
                            const int *ldb, int max_m, int max_n, const int *off, int *cursor,
-                           int *perm)
+                           int *perm, const int *only)
 {
   for (long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x; b < batch;
        b += (long long)gridDim.x * blockDim.x) {
+    if (only && !only[b]) continue;
     const int nn = n[b], mm = m[b], la = lda[b], lb = ldb[b];
     const bool ok = mm >= 0 && nn >= 1 && mm <= max_m && nn <= max_n && la >= nn &&
                     lb >= (mm > 1 ? mm : 1);
@@ -109,7 +114,7 @@ size_t vbatch_ws_bytes(KBlasHandle *h, int max_n, long long batch, bool mixed) {
   PosvPlan panel, reg;
   int st = mixed ? plan_vbatch<true>(h, max_n, panel, reg) : plan_vbatch<false>(h, max_n, panel, reg);
   if (st != KBLAS_Success) return 0;
-  return posv_ws_layout(max_n, batch, true, panel).total;
+  return posv_ws_layout(h, max_n, batch, true, !mixed && max_n > 32, panel).total;
 }
 
 // Uniform FP64 POSV / POTRF / POTRS (op 0 / 1 / 2) of order n > 32 on the
@@ -121,7 +126,7 @@ size_t fp64_uniform_ws_bytes(KBlasHandle *h, int n, long long batch) {
   if (n <= 32 || n > PC_MAX_N || batch <= 0) return 0;
   PosvPlan pl;
   if (plan_posv<false, 2>(h, n, pl) != KBLAS_Success) return 0;
-  return posv_ws_layout(n, batch, false, pl).total;
+  return posv_ws_layout(h, n, batch, false, true, pl).total;
 }
 
 int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, int batch,
@@ -130,7 +135,7 @@ int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, i
   PosvPlan pl;
   int st = plan_posv<false, 2>(h, n, pl);
   if (st != KBLAS_Success) return st;
-  const PosvWs ws = posv_ws_layout(n, batch, false, pl);
+  const PosvWs ws = posv_ws_layout(h, n, batch, false, true, pl);
   if (ws.total > h->ws.allocated.d_data_bytes || !h->ws.d_data) return KBLAS_InsufficientWorkspace;
   char *base = static_cast<char *>(h->ws.d_data);
   int *header = reinterpret_cast<int *>(base + ws.header);
@@ -139,12 +144,21 @@ int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, i
   sys.n = n;
   sys.m = (op == 1) ? 0 : m;
   sys.op = (op == 2) ? 2 : 0;
+  FixArgs fa{};
+  fa.info = info;
+  fa.redo_count = header + 1;
+  fa.redo_list = reinterpret_cast<int *>(base + ws.redo);
+  fa.scratch = reinterpret_cast<double *>(base + ws.scratch);
+  st = fix_launch(h, n, batch, sys, fa, header + 16);
+  if (st != KBLAS_Success || op == 2) return st;
+  // what the fixed-point kernel left: FP64
   ItemArgs it{};
-  it.uniform = 1;
-  it.batch = batch;
+  it.uniform = 2;
   it.n_uniform = n;
+  it.perm = fa.redo_list;
+  it.nitems_p = header + 1;
   it.queue = header;
-  OutArgs out{op == 2 ? nullptr : info, nullptr, base + ws.scratch, (long long)pl.slot_bytes,
+  OutArgs out{info, nullptr, base + ws.scratch, (long long)pl.slot_bytes,
               0, h->d_status};
   posv_persistent_kernel<false, 2><<<pl.grid, PC_NT, pl.smem, h->stream>>>(sys, it, out, pl.cfg, pl.smem);
   KGB_LAUNCH_CHECK("posv_persistent_kernel<fp64>");
@@ -171,7 +185,8 @@ static int vbatch(KBlasHandle *h, char side, char uplo, int *m, int *n, int max_
   PosvPlan pl, preg;
   int st = plan_vbatch<MIXED>(h, max_n, pl, preg);
   if (st != KBLAS_Success) return st;
-  const PosvWs ws = posv_ws_layout(max_n, batch, true, pl);
+  const bool fix = !MIXED && max_n > 32;
+  const PosvWs ws = posv_ws_layout(h, max_n, batch, true, fix, pl);
   if (ws.total > h->ws.allocated.d_data_bytes || !h->ws.d_data) return KBLAS_InsufficientWorkspace;
   char *base = static_cast<char *>(h->ws.d_data);
   int *header = reinterpret_cast<int *>(base + ws.header);
@@ -181,19 +196,27 @@ static int vbatch(KBlasHandle *h, char side, char uplo, int *m, int *n, int max_
   int *cursor = reinterpret_cast<int *>(base + ws.cursor);
   int *perm = reinterpret_cast<int *>(base + ws.perm);
   int4 *items = reinterpret_cast<int4 *>(base + ws.items);
-  // header .. cursor are contiguous: one memset clears them
-  cudaError_t e = cudaMemsetAsync(base, 0, ws.perm, h->stream);
-  if (e != cudaSuccess) return cuda_check(e, "cudaMemsetAsync", __FILE__, __LINE__);
+  int *redo = fix ? reinterpret_cast<int *>(base + ws.redo) : nullptr;
   const int tpb = 256;
   long long nb = (batch + tpb - 1) / tpb;
   const int blocks = (int)(nb < 4L * h->sm_count * 8 ? nb : 4L * h->sm_count * 8);
-  vb_count<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, cnt, info,
-                                          MIXED ? iter : nullptr);
-  KGB_LAUNCH_CHECK("vb_count");
-  vb_plan<<<1, 256, 0, h->stream>>>(max_n, cnt, off, ioff, items, header, pl.cfg);
-  KGB_LAUNCH_CHECK("vb_plan");
-  vb_scatter<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, off, cursor, perm);
-  KGB_LAUNCH_CHECK("vb_scatter");
+  // sort the systems (only: those marked) by order into perm and items; one
+  // memset clears header .. cursor and, the first time, the marks
+  auto sort = [&](const int *only) -> int {
+    cudaError_t e = cudaMemsetAsync(base, 0, only ? ws.redo : ws.perm, h->stream);
+    if (e != cudaSuccess) return cuda_check(e, "cudaMemsetAsync", __FILE__, __LINE__);
+    vb_count<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, cnt, info,
+                                            MIXED ? iter : nullptr, only);
+    KGB_LAUNCH_CHECK("vb_count");
+    vb_plan<<<1, 256, 0, h->stream>>>(max_n, cnt, off, ioff, items, header, pl.cfg);
+    KGB_LAUNCH_CHECK("vb_plan");
+    vb_scatter<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, off, cursor,
+                                              perm, only);
+    KGB_LAUNCH_CHECK("vb_scatter");
+    return KBLAS_Success;
+  };
+  st = sort(nullptr);
+  if (st != KBLAS_Success) return st;
   SysArgs sys{};
   sys.mode = 2;
   sys.Aarr = A;
@@ -211,7 +234,28 @@ static int vbatch(KBlasHandle *h, char side, char uplo, int *m, int *n, int max_
   it.split_p = header + 3;
   OutArgs out{info, MIXED ? iter : nullptr, base + ws.scratch, (long long)pl.slot_bytes,
               pl.tc, h->d_status};
-  // orders > 32 first (largest first), then orders <= 32 on the register path
+  auto small_orders = [&]() -> int {
+    it.queue = header + 2;
+    posv_persistent_kernel<MIXED, 1><<<preg.grid, PC_NT, preg.smem, h->stream>>>(sys, it, out, preg.cfg, preg.smem);
+    KGB_LAUNCH_CHECK("posv_persistent_kernel");
+    return KBLAS_Success;
+  };
+  // orders > 32 first (largest first), then orders <= 32 on the register path;
+  // plain FP64: in fixed point, and what that leaves on the FP64 panel path
+  if (fix) {
+    FixArgs fa{};
+    fa.off = off;
+    fa.cnt = cnt;
+    fa.perm = perm;
+    fa.narr = n;
+    fa.info = info;
+    fa.redo_mark = redo;
+    fa.scratch = reinterpret_cast<double *>(base + ws.scratch);
+    st = fix_launch(h, max_n, batch, sys, fa, header + 16);
+    if (st == KBLAS_Success) st = small_orders();
+    if (st == KBLAS_Success) st = sort(redo);
+    if (st != KBLAS_Success) return st;
+  }
   if (max_n > 32) {
     it.queue = header;
     bool launched = false;
@@ -225,10 +269,7 @@ static int vbatch(KBlasHandle *h, char side, char uplo, int *m, int *n, int max_
       posv_persistent_kernel<MIXED, 2><<<pl.grid, PC_NT, pl.smem, h->stream>>>(sys, it, out, pl.cfg, pl.smem);
     KGB_LAUNCH_CHECK("posv_persistent_kernel");
   }
-  it.queue = header + 2;
-  posv_persistent_kernel<MIXED, 1><<<preg.grid, PC_NT, preg.smem, h->stream>>>(sys, it, out, preg.cfg, preg.smem);
-  KGB_LAUNCH_CHECK("posv_persistent_kernel");
-  return KBLAS_Success;
+  return fix ? KBLAS_Success : small_orders();
 }
 
 }  // namespace kgb

@@ -6,9 +6,11 @@
 // flag support and return codes). Unlike the reference (host recursion over
 // TRSM + SYRK + cuBLAS GEMM, 4 launches at n = 32 and one HBM pass per level),
 // every call is ONE kernel launch: for n <= 32 the team kernel (POTRS of real
-// types: the register kernel, chol_reg.cuh) and, above,
-// the persistent panel kernel (double precision, when the workspace the
-// wsqueries request is allocated) or the blocked panel kernel (see
+// types: the register kernel, chol_reg.cuh; FP64 POTRF / POSV from order 17: the
+// fixed-point kernel, fix_kernel.cuh) and, above,
+// the fixed-point kernels (double precision, when the workspace the
+// wsqueries request is allocated; what does not fit fixed point goes on to the
+// persistent FP64 panel kernel) or the blocked panel kernel (see
 // chol_kernels.cuh).
 #include <stdio.h>
 #include <type_traits>
@@ -78,6 +80,20 @@ static int launch_blocked_nb(KBlasHandle *h, int n, int m, AccA A, int lda, AccB
   return KBLAS_Success;
 }
 
+template <int MODE, class AccA, class AccB>
+static int launch_fix_small(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int ldb,
+                            long long batch, int *info) {
+  auto kern = fix_small_kernel<MODE, AccA, AccB>;
+  kern<<<(unsigned)batch, 32, fix_smem_bytes<1, true>(n), h->stream>>>(n, m, A, lda, B, ldb, info);
+  KGB_LAUNCH_CHECK("fix_small_kernel");
+  return KBLAS_Success;
+}
+
+// FP64 POTRF / POSV from this order to 32: in fixed point, a warp per system
+// (10,000 POTRF + POTRS of order 32 412 -> 274 us, 200 POSV of order 24 92 -> 33 us,
+// copies of the operands included). Below, half of the warp's lanes would idle.
+constexpr int FIX_SMALL_MIN = 17;
+
 template <typename T, int MODE, class AccA, class AccB>
 static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int ldb,
                        long long batch, int *info) {
@@ -92,6 +108,10 @@ static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, in
     if (n <= 8) return launch_potrs_reg<T, 8>(h, n, m, A, lda, B, ldb, batch);
     if (n <= 16) return launch_potrs_reg<T, 16>(h, n, m, A, lda, B, ldb, batch);
     if (n <= 32) return launch_potrs_reg<T, 32>(h, n, m, A, lda, B, ldb, batch);
+  }
+  if constexpr (MODE != MODE_POTRS && std::is_same<T, double>::value) {
+    if (n >= FIX_SMALL_MIN && n <= 32)
+      return launch_fix_small<MODE>(h, n, m, A, lda, B, ldb, batch, info);
   }
   if (n <= 32) {
     switch (team_size_for(n, std::is_same<T, double>::value)) {
@@ -113,10 +133,10 @@ static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, in
   return KBLAS_NotSupported;
 }
 
-// Uniform FP64 orders 33..1024 go to the persistent panel path when the
-// handle's workspace covers it (posv_vbatch.cu; the wsqueries request it): for
-// 33 <= n <= 192 it is 1.3-2.9x faster than the one-launch blocked kernel
-// below, which remains the path when no workspace was allocated.
+// Uniform FP64 orders 33..1024 go to the fixed-point kernels (posv_fix.cu; what
+// does not fit them to the persistent FP64 panel kernel) when the handle's
+// workspace covers it (the wsqueries request it); the one-launch blocked kernel
+// below remains the path when no workspace was allocated.
 size_t fp64_uniform_ws_bytes(KBlasHandle *h, int n, long long batch);
 int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, int batch, int *info);
 
