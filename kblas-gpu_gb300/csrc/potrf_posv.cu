@@ -19,6 +19,7 @@
 
 #include "chol_kernels.cuh"
 #include "chol_reg.cuh"
+#include "chol_row.cuh"
 #include "kblas_internal.h"
 #include "launch_util.h"
 #include "posv_launch.h"
@@ -89,6 +90,18 @@ static int launch_fix_small(KBlasHandle *h, int n, int m, AccA A, int lda, AccB 
   return KBLAS_Success;
 }
 
+template <int NW, int R, int MODE, class AccA, class AccB>
+static int launch_row(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int ldb,
+                      long long batch, int *info) {
+  auto kern = chol_row_kernel<NW, R, MODE, AccA, AccB>;
+  const size_t smem = row_smem_bytes<NW>(n);
+  int st = set_smem(kern, smem);
+  if (st != KBLAS_Success) return st;
+  kern<<<(unsigned)batch, 32 * NW, smem, h->stream>>>(n, m, A, lda, B, ldb, info);
+  KGB_LAUNCH_CHECK("chol_row_kernel");
+  return KBLAS_Success;
+}
+
 // FP64 POTRF / POSV from this order to 32: in fixed point, a warp per system
 // (10,000 POTRF + POTRS of order 32 412 -> 274 us, 200 POSV of order 24 92 -> 33 us,
 // copies of the operands included). Below, half of the warp's lanes would idle.
@@ -121,6 +134,17 @@ static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, in
     }
   }
   const int limit = max_smem(h);
+  if constexpr (std::is_same<T, float>::value) {
+    // FP32 factors that fit in shared memory (order 330): one row per lane. As
+    // few warps as hold the rows, four to a lane: the fewer, the fewer loads of
+    // the pivot rows.
+    if (n <= row_max_n<4, 4>() && (long long)row_smem_bytes<4>(n) <= limit) {
+      if (n <= row_max_n<1, 2>()) return launch_row<1, 2, MODE>(h, n, m, A, lda, B, ldb, batch, info);
+      if (n <= row_max_n<1, 4>()) return launch_row<1, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
+      if (n <= row_max_n<2, 4>()) return launch_row<2, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
+      return launch_row<4, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
+    }
+  }
   int rc = (MODE == MODE_POTRF) ? 0 : (m < 8 ? m : 8);
   size_t s32 = blocked_smem_elems<T, 32, 32>(n, rc) * sizeof(T);
   if ((long long)s32 <= limit)
