@@ -1,22 +1,25 @@
 // chol_fix.cuh -- FP64 Cholesky in 64-bit fixed point on the integer pipe, and
 // the FP64 triangular solves with its factor (panel path, n > 32).
 //
-// Why: the part retires 2 FP64 FMA lanes per clock and SM but about 30 lanes of
-// a 32 x 32 -> 64-bit integer multiply-add, and three of those make a product
-// of two 60-bit numbers. A Cholesky factor suits fixed point: row i of L is
-// bounded by sqrt(a_ii), so its scale 2^E_i > sqrt(a_ii) is known beforehand.
+// Why: the part retires 2 FP64 FMA lanes per clock and SM, but 30 lanes of a 32 x
+// 32 -> 64-bit integer multiply-add and 64 or more of an FP32 FMA, and one of the
+// former with two of the latter make a product of two 56-bit numbers. A Cholesky
+// factor suits fixed point: row i of L is bounded by sqrt(a_ii), so its scale
+// 2^E_i > sqrt(a_ii) is known beforehand.
 //
-//   L(i, k) = X 2^(E_i - 59),  X = hi 2^30 + lo, |X| < 2^59, lo in [-2^29, 2^29)
+//   L(i, k) = X 2^(E_i - 56),  X = h 2^25 + l, |X| < 2^56, l in [-2^24, 2^24)
 //   S(i, j) = a_ij - sum_k L(i, k) L(j, k) in units of 2^(E_i + E_j - 62)
 //
-// A product adds hi hi' to one 64-bit sum and hi lo' + lo hi' to another (lo lo'
-// is below 2^-60 of the scales). The sums cannot overflow: sum |hi|^2 of a row
-// is at most 2^58 (Cauchy-Schwarz), so |sum hi hi'| <= 2^58 and
-// |sum hi lo' + lo hi'| <= 2 2^29 sqrt(K) 2^29: for
-// K = FX_FOLD = 128 columns, after which the sums are folded, <= 2^62.6. The pivot's reciprocal square root
-// (FP32 seed, one cubic step) and the scaling of a column are 64-bit integer
-// work too. The backward error |dA_ij| is a few 2^-60 sqrt(K) sqrt(a_ii a_jj),
-// below that of a chain of FP64 FMAs (bound K 2^-53 sqrt(a_ii a_jj)).
+// The products h h' are summed exactly in 64 bits: sum |h|^2 of a row is below
+// 2^62 (Cauchy-Schwarz). The products h l' + l h', 2^-32 of the scales, are summed
+// in FP32 (l is exact in FP32, h rounded to 24 bits) and join the 64-bit sum every
+// FX_FOLD = 16 columns, so that their roundings stay 2^-24 of 2^-31 of the scales;
+// l l' is below 2^-64. The pivot's reciprocal square root (FP32 seed, one cubic
+// step) and the scaling of a column are 64-bit integer work. Measured against quad
+// precision on shifted, conditioned and covariance matrices of order 33..400, the
+// errors of L and of the solutions are 0.3..1.0 times those of FP64 FMAs. The
+// backward error |dA_ij| is a few 2^-57 sqrt(K) sqrt(a_ii a_jj) (bound of a chain of
+// FP64 FMAs: K 2^-53 sqrt(a_ii a_jj)).
 //
 // A matrix that does not fit the scheme -- a pivot below 2^-42 a_jj, an entry
 // or a row of L above its bound (only when A is not positive definite), an
@@ -27,7 +30,7 @@
 // Work split: left-looking by blocks of 8 columns, one matrix row per lane (or
 // two): a lane keeps the 8 pairs of sums of each of its rows, loads its own
 // X(i, k) (8 bytes, lanes consecutive) and the 8 pivot rows' X(C + c, k) as four
-// 128-bit broadcasts: 24 (48) multiply-adds for 5 (6) loads. Lanes 0..7 of every
+// 128-bit broadcasts: 24 (48) products for 5 (6) loads. Lanes 0..7 of every
 // warp hold the block's 8 pivot rows, so each warp finds the pivots by itself:
 // the chain of 8 pivots, which the other warps would have to wait for, costs
 // every warp 8 lanes instead, and a block needs one barrier.
@@ -39,7 +42,7 @@
 namespace kgb {
 
 constexpr int FX_W = 8;         // columns per block
-constexpr int FX_FOLD = 128;    // columns after which the sums are folded
+constexpr int FX_FOLD = 16;     // columns after which the FP32 sums are folded
 constexpr int FX_DMIN_LOG = 20; // smallest pivot taken, in units of 2^(2 E - 62)
 
 // The lower triangle in blocks of 8 columns: block b holds the rows 8 b .. of
@@ -89,8 +92,10 @@ __device__ __forceinline__ long long fx_from(double a, int es, int &bad) {
   return (m ^ s) - s;
 }
 
-__device__ __forceinline__ long long fx_fold(long long hh, long long mid) {
-  return (long long)((unsigned long long)hh << 4) + ((mid + (1ll << 25)) >> 26);
+// The FP32 sum of h l' + l h' (units of 2^25 of those of S) joins hh.
+__device__ __forceinline__ void fx_fold(long long &hh, float &lo) {
+  hh += (long long)__float2int_rn(lo * 1.862645149230957e-9f) * 16;  // 2^-29
+  lo = 0.f;
 }
 
 // Reciprocal square root of a pivot: rho = rh 2^31 + rl = 2^92 / sqrt(d 4^z), z
@@ -100,7 +105,7 @@ struct FixPivot {
 };
 // Pivots and the pivot rows of the block at hand, one copy per warp.
 struct FixScratch {
-  double yd[FX_W][FX_W];  // limbs, [column][row]
+  double yd[FX_W][FX_W];  // [column][row]
   FixPivot pv[FX_W];
 };
 
@@ -130,7 +135,7 @@ __device__ __forceinline__ FixPivot fx_rsqrt(long long d) {
   return p;
 }
 
-// s rho 2^(z - 64): the entry of L in units of 2^(E - 59). bad gets set bits if s
+// s rho 2^(z - 67): the entry of L in units of 2^(E - 56). bad gets set bits if s
 // or the entry is out of range (the row's squares then exceed a_ii).
 __device__ __forceinline__ long long fx_scale_entry(long long s, const FixPivot &p, unsigned &bad) {
   const int sh = (int)(s >> 32);
@@ -139,38 +144,41 @@ __device__ __forceinline__ long long fx_scale_entry(long long s, const FixPivot 
   const int th = (int)(t >> 31), tl = (int)t & 0x7fffffff;
   long long m = (long long)th * p.rl;
   m += (long long)tl * p.rh;
-  long long x = (m >> 31) + 2;
+  long long x = (m >> 31) + 16;
   x += (long long)th * p.rh;
-  x >>= 2;
+  x >>= 5;
   const int xh = (int)(x >> 32);
-  bad |= (unsigned)(xh ^ (xh >> 31)) >> 27;
+  bad |= (unsigned)(xh ^ (xh >> 31)) >> 24;
   return x;
 }
 
-// Both limbs as the words of a double (never used as a floating-point value).
+// h and l (as FP32) as the words of a double (never used as a floating-point
+// value).
 __device__ __forceinline__ double fx_pack(long long x) {
-  const int lo = (int)((unsigned)x << 2) >> 2;
-  return __hiloint2double((int)((x - lo) >> 30), lo);
+  const int l = (int)((unsigned)x << 7) >> 7;
+  return __hiloint2double((int)((x - l) >> 25), __float_as_int((float)l));
 }
+__device__ __forceinline__ float fx_l(double v) { return __int_as_float(__double2loint(v)); }
 __device__ __forceinline__ long long fx_unpack(double v) {
-  return ((long long)__double2hiint(v) << 30) + __double2loint(v);
+  return ((long long)__double2hiint(v) << 25) + __float2int_rn(fx_l(v));
 }
-// The 8 products of x with y[c0..7], each kind of product in turn: the two that
-// share a sum are then 8 instructions apart.
-__device__ __forceinline__ void fx_mac(long long (&hh)[FX_W], long long (&mid)[FX_W], double x,
-                                       const double (&y)[FX_W], int c0) {
-  const int xh = __double2hiint(x), xl = __double2loint(x);
+
+// The 8 products of x with y[c0..7]; yf: FP32 of y's h.
+__device__ __forceinline__ void fx_mac(long long (&hh)[FX_W], float (&lo)[FX_W], double x,
+                                       const double (&y)[FX_W], const float (&yf)[FX_W], int c0) {
+  const int xh = __double2hiint(x);
+  const float xf = (float)xh, xl = fx_l(x);
 #pragma unroll
   for (int c = 0; c < FX_W; c++)
-    if (c >= c0) hh[c] += (long long)xh * __double2hiint(y[c]);
+    if (c >= c0) {
+      hh[c] += (long long)xh * __double2hiint(y[c]);
+      lo[c] = fmaf(xf, fx_l(y[c]), lo[c]);
+    }
 #pragma unroll
   for (int c = 0; c < FX_W; c++)
-    if (c >= c0) mid[c] += (long long)xh * __double2loint(y[c]);
-#pragma unroll
-  for (int c = 0; c < FX_W; c++)
-    if (c >= c0) mid[c] += (long long)xl * __double2hiint(y[c]);
+    if (c >= c0) lo[c] = fmaf(xl, yf[c], lo[c]);
 }
-// 8 consecutive limbs, 16-byte aligned
+// 8 consecutive elements, 16-byte aligned
 __device__ __forceinline__ void fx_ld8(const double *p, double (&y)[FX_W]) {
 #pragma unroll
   for (int c = 0; c < FX_W; c += 2) {
@@ -179,18 +187,23 @@ __device__ __forceinline__ void fx_ld8(const double *p, double (&y)[FX_W]) {
     y[c + 1] = v.y;
   }
 }
+__device__ __forceinline__ void fx_hf(const double (&y)[FX_W], float (&yf)[FX_W], int c0) {
+#pragma unroll
+  for (int c = 0; c < FX_W; c++)
+    if (c >= c0) yf[c] = (float)__double2hiint(y[c]);
+}
 
 // R rows of a thread against the block of columns C..C+7: the sums over the
-// columns before C (a: what was folded on the way is taken off).
+// columns before C.
 template <int R>
 __device__ __forceinline__ void fx_dot(const FixLayout &F, const double *Xs, int C,
                                        const int (&row)[R], long long (&hh)[R][FX_W],
-                                       long long (&mid)[R][FX_W], long long (&a)[R][FX_W])
+                                       float (&lo)[R][FX_W])
 {
 #pragma unroll
   for (int r = 0; r < R; r++)
 #pragma unroll
-    for (int c = 0; c < FX_W; c++) hh[r][c] = mid[r][c] = 0;
+    for (int c = 0; c < FX_W; c++) hh[r][c] = 0, lo[r][c] = 0.f;
   const double *P = Xs;
   int ld = F.n2;
   for (int K = 0; K < C; K += FX_W) {
@@ -199,13 +212,15 @@ __device__ __forceinline__ void fx_dot(const FixLayout &F, const double *Xs, int
 #pragma unroll 4
     for (int k = 0; k < FX_W; k++) {
       double y[FX_W], x[R];
+      float yf[FX_W];
       fx_ld8(yp, y);
+      fx_hf(y, yf, 0);
 #pragma unroll
       for (int r = 0; r < R; r++) x[r] = xp[row[r]];
       yp += ld;
       xp += ld;
 #pragma unroll
-      for (int r = 0; r < R; r++) fx_mac(hh[r], mid[r], x[r], y, 0);
+      for (int r = 0; r < R; r++) fx_mac(hh[r], lo[r], x[r], y, yf, 0);
     }
     P += FX_W * ld;
     ld -= FX_W;
@@ -213,10 +228,7 @@ __device__ __forceinline__ void fx_dot(const FixLayout &F, const double *Xs, int
 #pragma unroll
       for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int c = 0; c < FX_W; c++) {
-          a[r][c] -= fx_fold(hh[r][c], mid[r][c]);
-          hh[r][c] = mid[r][c] = 0;
-        }
+        for (int c = 0; c < FX_W; c++) fx_fold(hh[r][c], lo[r][c]);
     }
   }
 }
@@ -238,14 +250,13 @@ __device__ __forceinline__ void fx_copy8(double *dst, const double *src) {
 template <int R>
 __device__ __forceinline__ void fx_dot_staged(const FixLayout &F, const double *Xs, int C,
                                               const int (&row)[R], long long (&hh)[R][FX_W],
-                                              long long (&mid)[R][FX_W], long long (&a)[R][FX_W],
-                                              FixStage *st)
+                                              float (&lo)[R][FX_W], FixStage *st)
 {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int r = 0; r < R; r++)
 #pragma unroll
-    for (int c = 0; c < FX_W; c++) hh[r][c] = mid[r][c] = 0;
+    for (int c = 0; c < FX_W; c++) hh[r][c] = 0, lo[r][c] = 0.f;
   const double *P = Xs;  // the block to be copied next
   int ld = F.n2;
   auto copy = [&](int K) {
@@ -273,19 +284,18 @@ __device__ __forceinline__ void fx_dot_staged(const FixLayout &F, const double *
 #pragma unroll 2
     for (int k = 0; k < FX_W; k++) {
       double y[FX_W];
+      float yf[FX_W];
       fx_ld8(st->y[buf][k], y);
+      fx_hf(y, yf, 0);
 #pragma unroll
-      for (int r = 0; r < R; r++) fx_mac(hh[r], mid[r], st->x[buf][k][r * 32 + lane], y, 0);
+      for (int r = 0; r < R; r++) fx_mac(hh[r], lo[r], st->x[buf][k][r * 32 + lane], y, yf, 0);
     }
     __syncwarp();  // before this buffer is copied to again
     if (((K + FX_W) & (FX_FOLD - 1)) == 0) {
 #pragma unroll
       for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int c = 0; c < FX_W; c++) {
-          a[r][c] -= fx_fold(hh[r][c], mid[r][c]);
-          hh[r][c] = mid[r][c] = 0;
-        }
+        for (int c = 0; c < FX_W; c++) fx_fold(hh[r][c], lo[r][c]);
     }
   }
 }
@@ -299,7 +309,7 @@ template <int R, bool FIRST, bool KEEP>
 __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C,
                                            const int (&row)[R], const bool (&own)[R],
                                            int *zs, double *rho_s,
-                                           long long (&hh)[R][FX_W], long long (&mid)[R][FX_W],
+                                           long long (&hh)[R][FX_W], float (&lo)[R][FX_W],
                                            long long (&a)[R][FX_W], FixScratch *fs,
                                            float (&qs)[R], unsigned &bad)
 {
@@ -312,7 +322,10 @@ __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C
       long long s[R];
       FixPivot pv;
 #pragma unroll
-      for (int r = 0; r < R; r++) s[r] = a[r][c] - fx_fold(hh[r][c], mid[r][c]);
+      for (int r = 0; r < R; r++) {
+        fx_fold(hh[r][c], lo[r][c]);
+        s[r] = a[r][c] - hh[r][c];
+      }
       if (FIRST) {
         const long long d = __shfl_sync(0xffffffffu, s[0], c);
         if (d < (1ll << FX_DMIN_LOG) || d >= (1ll << 62)) return false;
@@ -343,9 +356,11 @@ __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C
         __syncwarp();
       }
       double y[FX_W];
+      float yf[FX_W];
       fx_ld8(fs->yd[c], y);
+      fx_hf(y, yf, c + 1);
 #pragma unroll
-      for (int r = 0; r < R; r++) fx_mac(hh[r], mid[r], x[r], y, c + 1);
+      for (int r = 0; r < R; r++) fx_mac(hh[r], lo[r], x[r], y, yf, c + 1);
     }
   }
   return true;
@@ -359,7 +374,8 @@ __device__ __forceinline__ bool fx_rows(const FixLayout &F, const double *A, int
                                         FixScratch *fs, FixStage *st, unsigned &bad)
 {
   int ri[R];
-  long long a[R][FX_W], hh[R][FX_W], mid[R][FX_W];
+  long long a[R][FX_W], hh[R][FX_W];
+  float lo[R][FX_W];
   {
     double av[R][FX_W];
     int b = 0;
@@ -378,19 +394,19 @@ __device__ __forceinline__ bool fx_rows(const FixLayout &F, const double *A, int
     }
     bad |= (unsigned)b;
   }
-  if (BIG) fx_dot_staged<R>(F, Xs, C, ri, hh, mid, a, st);
-  else fx_dot<R>(F, Xs, C, ri, hh, mid, a);
+  if (BIG) fx_dot_staged<R>(F, Xs, C, ri, hh, lo, st);
+  else fx_dot<R>(F, Xs, C, ri, hh, lo);
   float qs[R];
 #pragma unroll
   for (int r = 0; r < R; r++) qs[r] = 0.f;
-  const bool ok = fx_columns<R, FIRST, BIG>(F, Xs, C, row, own, zs, rho_s, hh, mid, a, fs, qs, bad);
+  const bool ok = fx_columns<R, FIRST, BIG>(F, Xs, C, row, own, zs, rho_s, hh, lo, a, fs, qs, bad);
   // a row whose squares add up to more than a_ii: A is not positive definite
 #pragma unroll
   for (int r = 0; r < R; r++)
     if (own[r]) {
       const float v = q[row[r]] + qs[r];
       q[row[r]] = v;
-      if (!(v < 288230376151711744.0f)) bad = 1;  // 2^58
+      if (!(v < 4611686018427387904.0f)) bad = 1;  // 2^62
     }
   return ok;
 }
@@ -432,7 +448,7 @@ __device__ __forceinline__ bool fx_block(const FixLayout &F, const double *A, in
   return ok;
 }
 
-// Cholesky factor of the lower triangle of A into Xs (limbs), by a CTA of NW
+// Cholesky factor of the lower triangle of A into Xs, by a CTA of NW
 // warps (n <= 8 + 56 NW, or BIG); rho_s, zs: the reciprocal roots of the pivots.
 // Es: n ints, q: n floats. False: the FP64 path has to take the matrix.
 // RMAX = 1: n <= 8 + 24 NW.
@@ -493,7 +509,7 @@ __device__ __forceinline__ int fx_potrf_fp64(const FixLayout &F, double *A, int 
   return 0;
 }
 
-// Limbs -> FP64, into A's lower triangle and (keep) in place; the reciprocals of
+// X -> FP64, into A's lower triangle and (keep) in place; the reciprocals of
 // the diagonal replace rho.
 template <int NW>
 __device__ __forceinline__ void fx_store(const FixLayout &F, double *Xs, const int *Es,
@@ -505,7 +521,7 @@ __device__ __forceinline__ void fx_store(const FixLayout &F, double *Xs, const i
   double *P = Xs;
   for (int C = 0; C < F.n; C += FX_W, P += FX_W * ld, ld -= FX_W) {
     for (int i = C + threadIdx.x; i < F.n; i += 32 * NW) {
-      const int e = Es[i] - 59;
+      const int e = Es[i] - 56;
       double *dst = A + (size_t)i + (size_t)C * lda, *src = P + (i - C);
       double v[FX_W];
       // (all loads before any store: the columns right of the diagonal, or of
@@ -575,13 +591,20 @@ __device__ __forceinline__ void fx_solve(const FixLayout &F, const T *Ps, const 
       const int i = s0 + j * RR + sub;
       y[j] = (on && i < n) ? b[(size_t)i * ldb] : T(0);
     }
+    // (rows past n repeat the last one: what they add up to is not used)
+    int ro[FX_NR];
+#pragma unroll
+    for (int j = 0; j < FX_NR; j++) ro[j] = min(s0 + j * RR + sub, n - 1);
 #pragma unroll 4
     for (int k = 0; k < s0; k++) {
-      const T *col = Ps + F.col(k) + (s0 + sub);
+      const T *col = Ps + F.col(k);
       const T yc = b[(size_t)k * ldb];
+      T l[FX_NR];
+#pragma unroll
+      for (int j = 0; j < FX_NR; j++) l[j] = col[ro[j]];
 #pragma unroll
       for (int j = 0; j < FX_NR; j++)
-        if (s0 + j * RR < n) y[j] -= ((s0 + j * RR + sub < n) ? col[j * RR] : T(0)) * yc;
+        if (s0 + j * RR < n) y[j] -= l[j] * yc;
     }
 #pragma unroll
     for (int jc = 0; jc < FX_NR; jc++) {
@@ -589,10 +612,9 @@ __device__ __forceinline__ void fx_solve(const FixLayout &F, const T *Ps, const 
       const int cn = min(RR, n - c0);
       T l[FX_NR];  // column c0 + c below its group; (PF) loaded ahead
       auto load = [&](int k) {
-        const T *col = Ps + F.col(k) + (c0 + sub);
+        const T *col = Ps + F.col(k);
 #pragma unroll
-        for (int j = jc; j < FX_NR; j++)
-          if (s0 + j * RR < n) l[j] = (s0 + j * RR + sub < n) ? col[(j - jc) * RR] : T(0);
+        for (int j = jc; j < FX_NR; j++) l[j] = col[ro[j]];
       };
       if (PF && cn > 0) load(c0);
       for (int c = 0; c < cn; c++) {
@@ -636,8 +658,11 @@ __device__ __forceinline__ void fx_solve(const FixLayout &F, const T *Ps, const 
 #pragma unroll 4
     for (int k = s0 + SEG; k < n; k++) {
       const T xc = b[(size_t)k * ldb];
+      T l[FX_NR];
 #pragma unroll
-      for (int j = 0; j < FX_NR; j++) y[j] -= Ps[off[j] + k] * xc;
+      for (int j = 0; j < FX_NR; j++) l[j] = Ps[off[j] + k];
+#pragma unroll
+      for (int j = 0; j < FX_NR; j++) y[j] -= l[j] * xc;
     }
 #pragma unroll
     for (int jc = FX_NR - 1; jc >= 0; jc--) {
@@ -682,7 +707,7 @@ __device__ __forceinline__ void fx_solve(const FixLayout &F, const T *Ps, const 
 // that leaves warps idle (an FMA of four costs the FP64 pipe the same as four of
 // one, but the chain of columns is walked once).
 template <int NW, bool PF, typename T>
-__device__ __forceinline__ void fx_solve_all(const FixLayout &F, const T *Ps, const T *rinv, T *B,
+__device__ __forceinline__ void fx_solve_all(FixLayout F, const T *Ps, const T *rinv, T *B,
                                              int ldb, int m)
 {
   const int w = threadIdx.x >> 5;

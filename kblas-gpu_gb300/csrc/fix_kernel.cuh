@@ -31,12 +31,13 @@ __host__ __device__ __forceinline__ size_t fix_smem_bytes(int n) {
 }
 
 // CTAs per SM that the registers are cut for: of one warp twelve (168 registers;
-// 20,000 systems of order 64 with 4 right-hand sides 1849 us, with eight, 255
-// registers, 2130), of two warps five (8,000 of order 80 1355 us, with four 1735)
-// or, with the factor in L2, the four that the scratch is for.
+// with eight, 255 registers, POSV of order 64 took 15% longer), of two warps five
+// (with four, 28% longer at order 80) or, with the factor in L2, the number that
+// the scratch is for: 8 warps to an SM (with 12, 168 registers, 25% longer at
+// order 200).
 template <int NW, bool FAC_SMEM>
 __host__ __device__ constexpr int fix_min_ctas() {
-  return NW == 1 ? 12 : FAC_SMEM ? 5 : 4;
+  return FAC_SMEM ? (NW == 1 ? 12 : 5) : 8 / NW;
 }
 
 // The solves as a function of their own: inlined, they and the factorization take
@@ -48,6 +49,15 @@ __device__ __noinline__ void fix_solve_smem(int n, int rinv_at, double *B, int l
   extern __shared__ __align__(16) unsigned char smem[];
   fx_solve_all<NW, false>(make_fix_layout(n), reinterpret_cast<const double *>(smem),
                           reinterpret_cast<const double *>(smem + rinv_at), B, ldb, m);
+}
+
+template <int NW>
+__device__ __noinline__ void fix_solve_l2(int n, const double *Xs, int rinv_at, double *B, int ldb,
+                                          int m)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  fx_solve_all<NW, true>(make_fix_layout(n), Xs, reinterpret_cast<const double *>(smem + rinv_at),
+                         B, ldb, m);
 }
 
 // POTRS: A holds the factor; m = 0: factor only.
@@ -104,10 +114,9 @@ fix_posv_kernel(SysArgs sys, FixArgs fa)
       }
     }
     if (ok && m > 0) {
-      if (FAC_SMEM)
-        fix_solve_smem<NW>(n, (int)(reinterpret_cast<unsigned char *>(rinv) - smem), B, ldb, m);
-      else
-        fx_solve_all<NW, true>(F, Xs, rinv, B, ldb, m);
+      const int rinv_at = (int)(reinterpret_cast<unsigned char *>(rinv) - smem);
+      if (FAC_SMEM) fix_solve_smem<NW>(n, rinv_at, B, ldb, m);
+      else fix_solve_l2<NW>(n, Xs, rinv_at, B, ldb, m);
     }
     fx_sync<NW>();
     if (uniform) q += gridDim.x;

@@ -149,6 +149,11 @@ struct ItemArgs {
   const int *nitems_p;  // number of items (device), binned batches
   const int *split_p;   // binned: items [0, *split_p) have n > 32, the rest n <= 32
   int *queue;           // work counter (zeroed before the launch)
+  // plain FP64: the launch shapes of a launch with few systems (more threads a
+  // system), taken when *few_p is not zero or, uniform 2, *nitems_p is at most few_max
+  const int *few_p;
+  int few_max;
+  PosvCfg few;
 };
 
 struct OutArgs {
@@ -717,6 +722,9 @@ posv_persistent_kernel(SysArgs sys, ItemArgs it, OutArgs out, PosvCfg cfg, int s
   }
   __syncthreads();
   if (use_tc) tc_fence_after_sync();
+  if constexpr (!MIXED && (PATHS & 2) != 0) {
+    if (it.uniform == 2 ? *it.nitems_p <= it.few_max : it.few_p && *it.few_p) cfg = it.few;
+  }
   TcCtx tcx{use_tc ? s_tmem : 0u, &s_tcbar, nullptr, &s_abort, out.status, 0u};
   long long first = 0, nitems;
   if (it.uniform) {

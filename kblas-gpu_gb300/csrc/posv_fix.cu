@@ -9,18 +9,18 @@ namespace kgb {
 
 // Orders lo < n <= hi and how a system of them runs. One warp holds 64 rows
 // (lanes 0..7 the pivots', 24 + 32 below them), two hold 120, so up to there a
-// block of columns passes over the rows once. The integer pipe wants 8 warps or
-// more on an SM: ten factors of order 64 fit into shared memory (21 KB each), four
-// of order 104; from there on the factors live in L2, which leaves four systems
-// of two warps to an SM whatever their order. us for 1 / 2 warps, then 1 / 2 / 4 / 8
-// with the factor in L2 (POSV, one right-hand side): 20,000 of order 64 1744 / 2326,
-// 3274 / 4221 / 5965 / 10998; 6,000 of 100 - / 2007, 2273 / 2697 / 4283 / 7432; 3,000
-// of 160 - / -, 3376 / 3087 / 4650 / 7372; 1,500 of 256 6203 / 5274 / 5967 / 8823.
+// block of columns passes over the rows once. Ten factors of order 64 fit into the
+// shared memory of an SM (19 KB each), four of order 104; larger ones live in L2,
+// eight systems of one warp to an SM (no barriers, and every warp busy to the last
+// column) until the systems of an SM no longer fit into its share of L2 and a
+// batch has fewer of them than warps: then four of two warps. us (POSV, one
+// right-hand side) for 2 warps in shared memory / 1 / 2 / 4 warps in L2: 6,000 of
+// order 100 1637 / 1745 / 2580 / 2687; 2,000 of 200 - / 2532 / 3481 / 3819; 1,500 of 256
+// - / 3777 / 4419 / 4761; 500 of 400 (4 right-hand sides) - / 5656 / 5078 / 5540.
 struct FixClass {
   int lo, hi;
 };
-constexpr int FIX_L2_WARPS = 2, FIX_L2_CTAS = 4;  // per system; CTAs per SM that the scratch is for
-static const FixClass FIX_CLASSES[FIX_NCLS] = {{32, 64}, {64, 104}, {104, PC_MAX_N}};
+static const FixClass FIX_CLASSES[FIX_NCLS] = {{32, 64}, {64, 104}, {104, 320}, {320, PC_MAX_N}};
 
 template <int NW, bool FAC_SMEM>
 static int launch_class(KBlasHandle *h, int hi, long long batch, const SysArgs &sys, FixArgs fa) {
@@ -33,7 +33,7 @@ static int launch_class(KBlasHandle *h, int hi, long long batch, const SysArgs &
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * NW, smem);
     if (e != cudaSuccess || per_sm < 1) per_sm = 1;
-    if (!FAC_SMEM && per_sm > FIX_L2_CTAS) per_sm = FIX_L2_CTAS;
+    if (!FAC_SMEM && per_sm > 8 / NW) per_sm = 8 / NW;  // as many as the scratch is for
     if (grid > (long long)h->sm_count * per_sm) grid = (long long)h->sm_count * per_sm;
   }
   kern<<<(unsigned)grid, 32 * NW, smem, h->stream>>>(sys, fa);
@@ -42,15 +42,20 @@ static int launch_class(KBlasHandle *h, int hi, long long batch, const SysArgs &
 }
 
 size_t fix_scratch_bytes(KBlasHandle *h, int max_n) {
-  if (max_n <= FIX_CLASSES[FIX_NCLS - 1].lo) return 0;
-  return (size_t)h->sm_count * FIX_L2_CTAS * make_fix_layout(max_n).total() * 8;
+  size_t most = 0;
+  for (int c = 2; c < FIX_NCLS; c++) {
+    const FixClass &k = FIX_CLASSES[c];
+    if (max_n <= k.lo) continue;
+    const size_t b = (size_t)(c == 2 ? 8 : 4) * make_fix_layout(max_n < k.hi ? max_n : k.hi).total() * 8;
+    if (b > most) most = b;
+  }
+  return most * h->sm_count;
 }
 
 int fix_launch(KBlasHandle *h, int max_n, long long batch, const SysArgs &sys, FixArgs fa,
                int *queues) {
   const bool uniform = fa.perm == nullptr;
   fa.batch = batch;
-  fa.slot = make_fix_layout(max_n).total();
   for (int c = FIX_NCLS - 1; c >= 0; c--) {
     const FixClass &k = FIX_CLASSES[c];
     if (max_n <= k.lo || (uniform && max_n > k.hi)) continue;
@@ -58,11 +63,13 @@ int fix_launch(KBlasHandle *h, int max_n, long long batch, const SysArgs &sys, F
     fa.lo = k.lo;
     fa.hi = hi;
     fa.queue = queues + c;
+    fa.slot = make_fix_layout(hi).total();
     int st;
     switch (c) {
       case 0: st = launch_class<1, true>(h, hi, batch, sys, fa); break;
       case 1: st = launch_class<2, true>(h, hi, batch, sys, fa); break;
-      default: st = launch_class<FIX_L2_WARPS, false>(h, hi, batch, sys, fa); break;
+      case 2: st = launch_class<1, false>(h, hi, batch, sys, fa); break;
+      default: st = launch_class<2, false>(h, hi, batch, sys, fa); break;
     }
     if (st != KBLAS_Success) return st;
   }

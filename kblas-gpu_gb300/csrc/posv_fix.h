@@ -6,7 +6,7 @@
 
 namespace kgb {
 
-constexpr int FIX_NCLS = 3;
+constexpr int FIX_NCLS = 4;
 
 // Bytes of scratch for orders up to max_n (after ensure_device_props).
 size_t fix_scratch_bytes(KBlasHandle *h, int max_n);

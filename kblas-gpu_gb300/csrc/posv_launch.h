@@ -67,6 +67,22 @@ static inline PosvCfg current_cfg(bool mixed) {
   return c;
 }
 
+// What the fixed-point kernels leave to the FP64 panel path is mostly a handful of
+// systems: with at most PC_FEW of them the time is one system's latency, so the
+// teams are wider (order 256: 64 -> 256 threads).
+constexpr int PC_FEW = 304;
+static inline PosvCfg few_cfg() {
+  PosvCfg c = default_cfg(false);
+  const int nmax[PC_NCLS] = {8, 16, 32, 64, 96, 128, 176, PC_MAX_N};
+  const int ts[PC_NCLS] = {8, 16, 32, 64, 128, 256, 256, 256};
+  for (int k = 0; k < PC_NCLS; k++) {
+    c.nmax[k] = nmax[k];
+    c.ts[k] = ts[k];
+    c.spi[k] = PC_NT / ts[k];
+  }
+  return c;
+}
+
 // A class whose orders are all <= 32 runs the register path: team size W in
 // {8, 16, 32} with W >= its largest order. A class with orders above 32 runs
 // the panel path: whole warps (32..256); one that straddles 32 needs W = 32.
@@ -89,8 +105,8 @@ static inline bool cfg_valid(const PosvCfg &c) {
 // shared memory = the largest need over the size classes that kernel serves
 // (register path: orders <= 32; panel path: orders > 32).
 template <bool MIXED, int PATHS = 3>
-static inline int plan_posv(KBlasHandle *h, int max_n, PosvPlan &pl) {
-  pl.cfg = current_cfg(MIXED);
+static inline int plan_posv(KBlasHandle *h, int max_n, PosvPlan &pl, const PosvCfg *cfg = nullptr) {
+  pl.cfg = cfg ? *cfg : current_cfg(MIXED);
   if (!cfg_valid(pl.cfg)) return KBLAS_WrongConfig;
   const size_t budget = (size_t)(max_smem(h) < (int)PC_SMEM_BUDGET ? max_smem(h) : (int)PC_SMEM_BUDGET);
   // shared memory of the launch: the largest need over the classes in range
@@ -140,13 +156,13 @@ static inline int plan_posv(KBlasHandle *h, int max_n, PosvPlan &pl) {
     if constexpr (MIXED && (PATHS & 2) != 0) {
       if (tc) {
         auto kern = posv_persistent_kernel<MIXED, PATHS | 4>;
-        st = set_smem(kern, bytes);
+        st = set_smem(kern, budget);
         if (st == KBLAS_Success) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PC_NT, bytes);
       }
     }
     if (!tc) {
       auto kern = posv_persistent_kernel<MIXED, PATHS>;
-      st = set_smem(kern, bytes);
+      st = set_smem(kern, budget);  // the same from every thread, whatever its orders
       if (st == KBLAS_Success) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PC_NT, bytes);
     }
     if (e != cudaSuccess || per_sm < 1) per_sm = 1;
@@ -167,6 +183,21 @@ static inline int plan_posv(KBlasHandle *h, int max_n, PosvPlan &pl) {
   pl.grid = h->sm_count * per_sm;
   pl.slot_bytes = (PATHS & 2) ? posv_slot_bytes(pl.cfg, max_n) : 0;
   return KBLAS_Success;
+}
+
+// The plan of the FP64 panel launch behind the fixed-point kernels: the tuning
+// table's, in a CTA that also holds few_cfg's teams.
+static inline int plan_redo(KBlasHandle *h, int max_n, PosvPlan &pl) {
+  int st = plan_posv<false, 2>(h, max_n, pl);
+  if (st != KBLAS_Success) return st;
+  PosvPlan few;
+  const PosvCfg c = few_cfg();
+  st = plan_posv<false, 2>(h, max_n, few, &c);
+  if (st != KBLAS_Success) return st;
+  if (few.smem > pl.smem) pl.smem = few.smem;
+  if (few.grid < pl.grid) pl.grid = few.grid;
+  if (few.slot_bytes > pl.slot_bytes) pl.slot_bytes = few.slot_bytes;
+  return st;
 }
 
 // Device workspace layout shared by the uniform mixed and the variable-size

@@ -52,9 +52,21 @@ __global__ void vb_count(long long batch, const int *n, const int *m, const int 
   }
 }
 
+// few, few_max: the shapes for at most few_max systems (header[4] tells the launch).
 __global__ void vb_plan(int max_n, const int *cnt, int *off, int *ioff, int4 *items, int *header,
-                        PosvCfg cfg)
+                        PosvCfg cfg, PosvCfg few, int few_max)
 {
+  __shared__ int s_few;
+  if (threadIdx.x == 0) s_few = 0;
+  __syncthreads();
+  int total = 0;
+  for (int nn = 1 + threadIdx.x; nn <= max_n; nn += blockDim.x) total += cnt[nn];
+  if (total) atomicAdd(&s_few, total);
+  __syncthreads();
+  const bool use_few = s_few <= few_max;
+  if (use_few) cfg = few;
+  if (threadIdx.x == 0) header[4] = use_few;
+
   // prefix sums over n, largest n first (max_n <= 1024: one thread suffices)
   if (threadIdx.x == 0) {
     int o = 0, io = 0, split = -1;
@@ -103,7 +115,7 @@ template <bool MIXED>
 static int plan_vbatch(KBlasHandle *h, int max_n, PosvPlan &panel, PosvPlan &reg) {
   int st = plan_posv<MIXED, 1>(h, max_n < 32 ? max_n : 32, reg);
   if (st != KBLAS_Success) return st;
-  if (max_n > 32) return plan_posv<MIXED, 2>(h, max_n, panel);
+  if (max_n > 32) return MIXED ? plan_posv<MIXED, 2>(h, max_n, panel) : plan_redo(h, max_n, panel);
   panel = reg;
   panel.slot_bytes = 0;
   return KBLAS_Success;
@@ -125,7 +137,7 @@ size_t vbatch_ws_bytes(KBlasHandle *h, int max_n, long long batch, bool mixed) {
 size_t fp64_uniform_ws_bytes(KBlasHandle *h, int n, long long batch) {
   if (n <= 32 || n > PC_MAX_N || batch <= 0) return 0;
   PosvPlan pl;
-  if (plan_posv<false, 2>(h, n, pl) != KBLAS_Success) return 0;
+  if (plan_redo(h, n, pl) != KBLAS_Success) return 0;
   return posv_ws_layout(h, n, batch, false, true, pl).total;
 }
 
@@ -133,7 +145,7 @@ int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, i
                             int *info) {
   if (n <= 32 || n > PC_MAX_N) return KBLAS_NotSupported;
   PosvPlan pl;
-  int st = plan_posv<false, 2>(h, n, pl);
+  int st = plan_redo(h, n, pl);
   if (st != KBLAS_Success) return st;
   const PosvWs ws = posv_ws_layout(h, n, batch, false, true, pl);
   if (ws.total > h->ws.allocated.d_data_bytes || !h->ws.d_data) return KBLAS_InsufficientWorkspace;
@@ -158,6 +170,8 @@ int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, i
   it.perm = fa.redo_list;
   it.nitems_p = header + 1;
   it.queue = header;
+  it.few_max = PC_FEW;
+  it.few = few_cfg();
   OutArgs out{info, nullptr, base + ws.scratch, (long long)pl.slot_bytes,
               0, h->d_status};
   posv_persistent_kernel<false, 2><<<pl.grid, PC_NT, pl.smem, h->stream>>>(sys, it, out, pl.cfg, pl.smem);
@@ -208,7 +222,8 @@ static int vbatch(KBlasHandle *h, char side, char uplo, int *m, int *n, int max_
     vb_count<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, cnt, info,
                                             MIXED ? iter : nullptr, only);
     KGB_LAUNCH_CHECK("vb_count");
-    vb_plan<<<1, 256, 0, h->stream>>>(max_n, cnt, off, ioff, items, header, pl.cfg);
+    vb_plan<<<1, 256, 0, h->stream>>>(max_n, cnt, off, ioff, items, header, pl.cfg, few_cfg(),
+                                      only ? PC_FEW : -1);
     KGB_LAUNCH_CHECK("vb_plan");
     vb_scatter<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, off, cursor,
                                               perm, only);
@@ -255,6 +270,8 @@ static int vbatch(KBlasHandle *h, char side, char uplo, int *m, int *n, int max_
     if (st == KBLAS_Success) st = small_orders();
     if (st == KBLAS_Success) st = sort(redo);
     if (st != KBLAS_Success) return st;
+    it.few_p = header + 4;
+    it.few = few_cfg();
   }
   if (max_n > 32) {
     it.queue = header;
