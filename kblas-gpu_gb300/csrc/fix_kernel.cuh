@@ -37,7 +37,7 @@ __host__ __device__ __forceinline__ size_t fix_smem_bytes(int n) {
 // order 200).
 template <int NW, bool FAC_SMEM>
 __host__ __device__ constexpr int fix_min_ctas() {
-  return FAC_SMEM ? (NW == 1 ? 12 : 5) : 8 / NW;
+  return FAC_SMEM ? (NW == 1 ? 12 : NW == 2 ? 5 : 1) : 8 / NW;
 }
 
 // The solves as a function of their own: inlined, they and the factorization take

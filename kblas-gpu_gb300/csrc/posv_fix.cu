@@ -21,12 +21,17 @@ struct FixClass {
   int lo, hi;
 };
 static const FixClass FIX_CLASSES[FIX_NCLS] = {{32, 64}, {64, 104}, {104, 320}, {320, PC_MAX_N}};
+// A batch of at most two systems per SM waits for single systems: above order 104
+// they get eight warps, the factor in shared memory up to 216 (197 KB). 50 of order
+// 200 1011 -> 358 us, of 400 2811 -> 2047 (two right-hand sides).
+static const FixClass FIX_FEW[FIX_NCLS] = {{32, 64}, {64, 104}, {104, 216}, {216, PC_MAX_N}};
 
 template <int NW, bool FAC_SMEM>
-static int launch_class(KBlasHandle *h, int hi, long long batch, const SysArgs &sys, FixArgs fa) {
+static int launch_class(KBlasHandle *h, int hi, int class_hi, long long batch, const SysArgs &sys,
+                        FixArgs fa) {
   auto kern = fix_posv_kernel<NW, FAC_SMEM>;
   const size_t smem = fix_smem_bytes<NW, FAC_SMEM>(hi);
-  int st = set_smem(kern, smem);
+  int st = set_smem(kern, fix_smem_bytes<NW, FAC_SMEM>(class_hi));  // the same from every thread
   if (st != KBLAS_Success) return st;
   long long grid = batch;
   if (!FAC_SMEM || fa.perm) {  // resident CTAs: their scratch, or their queue
@@ -54,10 +59,10 @@ size_t fix_scratch_bytes(KBlasHandle *h, int max_n) {
 
 int fix_launch(KBlasHandle *h, int max_n, long long batch, const SysArgs &sys, FixArgs fa,
                int *queues) {
-  const bool uniform = fa.perm == nullptr;
+  const bool uniform = fa.perm == nullptr, few = batch <= 2 * h->sm_count;
   fa.batch = batch;
   for (int c = FIX_NCLS - 1; c >= 0; c--) {
-    const FixClass &k = FIX_CLASSES[c];
+    const FixClass &k = few ? FIX_FEW[c] : FIX_CLASSES[c];
     if (max_n <= k.lo || (uniform && max_n > k.hi)) continue;
     const int hi = max_n < k.hi ? max_n : k.hi;
     fa.lo = k.lo;
@@ -66,10 +71,16 @@ int fix_launch(KBlasHandle *h, int max_n, long long batch, const SysArgs &sys, F
     fa.slot = make_fix_layout(hi).total();
     int st;
     switch (c) {
-      case 0: st = launch_class<1, true>(h, hi, batch, sys, fa); break;
-      case 1: st = launch_class<2, true>(h, hi, batch, sys, fa); break;
-      case 2: st = launch_class<1, false>(h, hi, batch, sys, fa); break;
-      default: st = launch_class<2, false>(h, hi, batch, sys, fa); break;
+      case 0: st = launch_class<1, true>(h, hi, k.hi, batch, sys, fa); break;
+      case 1: st = launch_class<2, true>(h, hi, k.hi, batch, sys, fa); break;
+      case 2:
+        st = few ? launch_class<8, true>(h, hi, k.hi, batch, sys, fa)
+                 : launch_class<1, false>(h, hi, k.hi, batch, sys, fa);
+        break;
+      default:
+        st = few ? launch_class<8, false>(h, hi, k.hi, batch, sys, fa)
+                 : launch_class<2, false>(h, hi, k.hi, batch, sys, fa);
+        break;
     }
     if (st != KBLAS_Success) return st;
   }

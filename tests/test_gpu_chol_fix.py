@@ -59,6 +59,19 @@ def test_block_edges(gpu, handle, kb, wl, n, array):
         check_factor(a, out, n, b)
 
 
+@pytest.mark.parametrize("n", [105, 128, 217, 319, 320, 321])
+def test_block_edges_many_systems(gpu, handle, kb, wl, n):
+    """More than two systems per SM: one or two warps a system, the factor in L2."""
+    few = make_batch(wl, 5, n, n, np.float64, seed=n)
+    a = np.ascontiguousarray(np.tile(few, (70, 1, 1)))
+    out, info = potrf(gpu, handle, kb, a, n, n)
+    assert (info == 0).all()
+    check_untouched(few, out[-5:], n)
+    for b in range(5):
+        check_factor(few, out, n, b)
+    assert np.array_equal(out, np.tile(out[:5], (70, 1, 1)))
+
+
 @pytest.mark.parametrize("data", ["cond", "cov", "graded", "huge", "tiny", "small_pivot"])
 @pytest.mark.parametrize("n", [24, 48, 131])
 def test_hard_data(gpu, handle, kb, wl, data, n):
