@@ -94,8 +94,9 @@ template <int NW, int R, int MODE, class AccA, class AccB>
 static int launch_row(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int ldb,
                       long long batch, int *info) {
   auto kern = chol_row_kernel<NW, R, MODE, AccA, AccB>;
-  const size_t smem = row_smem_bytes<NW>(n);
-  int st = set_smem(kern, smem);
+  const size_t smem = row_smem_bytes<NW>(n), most = row_smem_bytes<NW>(row_max_n<NW, R>());
+  const size_t limit = (size_t)max_smem(h);
+  int st = set_smem(kern, most < limit ? most : limit);  // the same from every thread
   if (st != KBLAS_Success) return st;
   kern<<<(unsigned)batch, 32 * NW, smem, h->stream>>>(n, m, A, lda, B, ldb, info);
   KGB_LAUNCH_CHECK("chol_row_kernel");
@@ -135,13 +136,15 @@ static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, in
   }
   const int limit = max_smem(h);
   if constexpr (std::is_same<T, float>::value) {
-    // FP32 factors that fit in shared memory (order 330): one row per lane. As
-    // few warps as hold the rows, four to a lane: the fewer, the fewer loads of
-    // the pivot rows.
+    // FP32 factors that fit in shared memory (order 330): one row per lane. One
+    // warp as long as it holds the rows, four to a lane (the fewer warps, the fewer
+    // loads of the pivot rows); above, four warps, as only two factors or one fit on
+    // an SM. us for 1 / 2 / 4 warps: 4,000 of order 100 237 / 313 / 297, 3,000 of 128
+    // 334 / 421 / 360, 1,500 of 200 - / 872 / 699.
     if (n <= row_max_n<4, 4>() && (long long)row_smem_bytes<4>(n) <= limit) {
       if (n <= row_max_n<1, 2>()) return launch_row<1, 2, MODE>(h, n, m, A, lda, B, ldb, batch, info);
       if (n <= row_max_n<1, 4>()) return launch_row<1, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
-      if (n <= row_max_n<2, 4>()) return launch_row<2, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
+      if (n <= row_max_n<4, 2>()) return launch_row<4, 2, MODE>(h, n, m, A, lda, B, ldb, batch, info);
       return launch_row<4, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
     }
   }
