@@ -52,6 +52,9 @@ __global__ void vb_count(long long batch, const int *n, const int *m, const int 
   }
 }
 
+constexpr int VB_PLAN_NT = 256;
+
+// One CTA of VB_PLAN_NT threads.
 // few, few_max: the shapes for at most few_max systems (header[4] tells the launch).
 __global__ void vb_plan(int max_n, const int *cnt, int *off, int *ioff, int4 *items, int *header,
                         PosvCfg cfg, PosvCfg few, int few_max)
@@ -67,20 +70,37 @@ __global__ void vb_plan(int max_n, const int *cnt, int *off, int *ioff, int4 *it
   if (use_few) cfg = few;
   if (threadIdx.x == 0) header[4] = use_few;
 
-  // prefix sums over n, largest n first (max_n <= 1024: one thread suffices)
-  if (threadIdx.x == 0) {
-    int o = 0, io = 0, split = -1;
-    for (int nn = max_n; nn >= 1; nn--) {
-      if (split < 0 && nn <= 32) split = io;  // items of orders > 32 come first
-      off[nn] = o;
-      ioff[nn] = io;
-      const int c = cnt[nn];
-      const int spi = cfg.spi[pc_class(cfg, nn)];
-      o += c;
-      io += (c + spi - 1) / spi;
-    }
-    header[1] = io;
-    header[3] = split < 0 ? io : split;
+  // prefix sums over n, largest n first: a thread takes `per` consecutive orders
+  // (a walk of one thread over 256 orders took 45 us, mostly waiting for loads; so
+  // 10 us)
+  __shared__ int s_sum[2][VB_PLAN_NT / 32];
+  const int per = (max_n + VB_PLAN_NT - 1) / VB_PLAN_NT;
+  const int top = max_n - threadIdx.x * per, end = max(top - per, 0);  // orders (end, top]
+  int o = 0, io = 0;
+  for (int nn = top; nn > end; nn--) {
+    const int c = cnt[nn], spi = cfg.spi[pc_class(cfg, nn)];
+    o += c;
+    io += (c + spi - 1) / spi;
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int po = o, pio = io;  // sums up to and including this thread's
+  for (int d = 1; d < 32; d <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, po, d), b = __shfl_up_sync(0xffffffffu, pio, d);
+    if (lane >= d) po += a, pio += b;
+  }
+  if (lane == 31) s_sum[0][w] = po, s_sum[1][w] = pio;
+  __syncthreads();
+  for (int k = 0; k < w; k++) po += s_sum[0][k], pio += s_sum[1][k];
+  if (threadIdx.x == VB_PLAN_NT - 1) header[1] = pio;
+  o = po - o;
+  io = pio - io;
+  for (int nn = top; nn > end; nn--) {
+    const int c = cnt[nn], spi = cfg.spi[pc_class(cfg, nn)];
+    off[nn] = o;
+    ioff[nn] = io;
+    if (nn == min(32, max_n)) header[3] = io;  // items of orders > 32 come first
+    o += c;
+    io += (c + spi - 1) / spi;
   }
   __syncthreads();
   for (int nn = 1 + threadIdx.x; nn <= max_n; nn += blockDim.x) {
@@ -222,7 +242,7 @@ static int vbatch(KBlasHandle *h, char side, char uplo, int *m, int *n, int max_
     vb_count<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, cnt, info,
                                             MIXED ? iter : nullptr, only);
     KGB_LAUNCH_CHECK("vb_count");
-    vb_plan<<<1, 256, 0, h->stream>>>(max_n, cnt, off, ioff, items, header, pl.cfg, few_cfg(),
+    vb_plan<<<1, VB_PLAN_NT, 0, h->stream>>>(max_n, cnt, off, ioff, items, header, pl.cfg, few_cfg(),
                                       only ? PC_FEW : -1);
     KGB_LAUNCH_CHECK("vb_plan");
     vb_scatter<<<blocks, tpb, 0, h->stream>>>(batch, n, m, lda, ldb, max_m, max_n, off, cursor,
