@@ -665,11 +665,18 @@ __device__ __forceinline__ void item_decode(const ItemArgs &it, const PosvCfg &c
   }
 }
 
+// The system at a slot of the item table (mixed launches have no listed systems).
+template <bool MIXED>
+__device__ __forceinline__ long long item_system(const ItemArgs &it, int slot) {
+  return (MIXED ? it.uniform != 0 : it.uniform == 1) ? (long long)slot : (long long)it.perm[slot];
+}
+
 // Ask L2 for the lower triangles of the next item's matrices while the
 // current item is being processed, so the next item's staging loads hit L2
 // instead of waiting on HBM: one TMA bulk prefetch per column (rows j..n-1,
 // contiguous), trimmed inward to 16-byte boundaries as the bulk operation
 // requires, so it never reaches outside the column's own range.
+template <bool MIXED>
 __device__ __forceinline__ void prefetch_item(const SysArgs &sys, const ItemArgs &it,
                                               const PosvCfg &cfg, long long q) {
   int n, start, count;
@@ -677,7 +684,7 @@ __device__ __forceinline__ void prefetch_item(const SysArgs &sys, const ItemArgs
   const int pairs = count * n;  // (system, column) pairs
   for (int pc = threadIdx.x; pc < pairs; pc += blockDim.x) {
     const int k = pc / n, j = pc - k * n;
-    const long long sidx = it.uniform == 1 ? (long long)start + k : (long long)it.perm[start + k];
+    const long long sidx = item_system<MIXED>(it, start + k);
     int m, lda, ldb;
     double *A, *B;
     sys.get(sidx, m, A, lda, B, ldb);
@@ -728,7 +735,9 @@ posv_persistent_kernel(SysArgs sys, ItemArgs it, OutArgs out, PosvCfg cfg, int s
   TcCtx tcx{use_tc ? s_tmem : 0u, &s_tcbar, nullptr, &s_abort, out.status, 0u};
   long long first = 0, nitems;
   if (it.uniform) {
-    if (it.uniform == 2) it.batch = *it.nitems_p;
+    if constexpr (!MIXED) {  // (the mixed kernels' parameters stay where they are)
+      if (it.uniform == 2) it.batch = *it.nitems_p;
+    }
     const int spi = cfg.spi[pc_class(cfg, it.n_uniform)];
     nitems = (it.batch + spi - 1) / spi;
   } else {
@@ -748,7 +757,7 @@ posv_persistent_kernel(SysArgs sys, ItemArgs it, OutArgs out, PosvCfg cfg, int s
     // claim the next item now and warm L2 with its matrices
     if (threadIdx.x == 0) s_item = (int)first + atomicAdd(it.queue, 1);
     __syncthreads();
-    if (s_item < nitems) prefetch_item(sys, it, cfg, s_item);
+    if (s_item < nitems) prefetch_item<MIXED>(sys, it, cfg, s_item);
     int n, start, count;
     item_decode(it, cfg, q, n, start, count);
     const int c = pc_class(cfg, n);
@@ -764,7 +773,7 @@ posv_persistent_kernel(SysArgs sys, ItemArgs it, OutArgs out, PosvCfg cfg, int s
     int m = 0, lda = 1, ldb = 1;
     double *A = nullptr, *B = nullptr;
     if (active) {
-      sidx = it.uniform == 1 ? (long long)start + team_id : (long long)it.perm[start + team_id];
+      sidx = item_system<MIXED>(it, start + team_id);
       sys.get(sidx, m, A, lda, B, ldb);
     }
     unsigned char *base = smem + (size_t)team_id * tb;
