@@ -141,7 +141,13 @@ static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, in
     // loads of the pivot rows); above, four warps, as only two factors or one fit on
     // an SM. us for 1 / 2 / 4 warps: 4,000 of order 100 237 / 313 / 297, 3,000 of 128
     // 334 / 421 / 360, 1,500 of 200 - / 872 / 699.
-    if (n <= row_max_n<4, 4>() && (long long)row_smem_bytes<4>(n) <= limit) {
+    // POTRS alone stays with the blocked kernel above order 200: there is no
+    // factorization to pay for bringing the factor in by one or two CTAs on an SM.
+    // POTRF + POTRS, us with the row kernel in both, with it in POTRF alone, and in
+    // neither: 600 of order 250 1241 / 907 / 1010, 1,500 of 150 555 / - / 1134,
+    // 800 of 200 757 / - / 1106.
+    if (n <= (MODE == MODE_POTRS ? 200 : row_max_n<4, 4>()) &&
+        (long long)row_smem_bytes<4>(n) <= limit) {
       if (n <= row_max_n<1, 2>()) return launch_row<1, 2, MODE>(h, n, m, A, lda, B, ldb, batch, info);
       if (n <= row_max_n<1, 4>()) return launch_row<1, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
       if (n <= row_max_n<4, 2>()) return launch_row<4, 2, MODE>(h, n, m, A, lda, B, ldb, batch, info);
