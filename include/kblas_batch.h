@@ -43,11 +43,12 @@ typedef struct KBlasHandle *kblasHandle_t;
  * workspace to what the routine needs; kblasAllocateWorkspace then allocates.
  * SYRK, TRSM and TRMM need none (zero-byte requests, kept so KBLAS callers
  * link unchanged). The double-precision POTRF / POTRS / POSV of order 33..1024
- * request scratch for the persistent panel kernel and run on it once the
- * workspace is allocated; without it they run on a one-launch blocked kernel
- * that needs none but is several times slower at small orders (about 14% of
- * the FP64 peak at n = 64 against 33% with the workspace). Call the query and
- * kblasAllocateWorkspace, as KBLAS callers do, before timing these routines.
+ * request scratch for the fixed-point kernels and the FP64 panel kernel behind
+ * them and run on these once the workspace is allocated; without it they run
+ * on a one-launch blocked kernel that needs none but is many times slower
+ * (about 14% of the FP64 peak at n = 64 against 110% with the workspace). Call
+ * the query and kblasAllocateWorkspace, as KBLAS callers do, before timing
+ * these routines.
  * ------------------------------------------------------------------------- */
 void kblas_syrk_batch_wsquery(kblasHandle_t handle, const int m, int batchCount);
 void kblas_trsm_batch_wsquery(kblasHandle_t handle, char side, int m, int n, int batchCount);
@@ -459,11 +460,11 @@ int kblasDposv_batch_mixed(kblasHandle_t handle, char side, char uplo,
                            double **A_array, int lda, double **B_array, int ldb,
                            int batchCount, int *info_array, int *iter_array);
 
-/* Variable-size POSV in one persistent launch. m, n, lda, ldb are DEVICE
+/* Variable-size POSV in a few launches. m, n, lda, ldb are DEVICE
  * int[batchCount] (the non-uniform convention of reference
  * include/kblas_batch.h:829-845); max_m / max_n bound them. Matrices are
- * binned by size class on the device, then one persistent kernel pulls work
- * items from a device queue, factorizes, solves and (for _mixed) refines each
+ * binned by size class on the device, then persistent kernels pull work
+ * items from device queues, factorize, solve and (for _mixed) refine each
  * system while it is resident on chip. No host synchronisation: the sequence
  * can be captured in a CUDA graph. Needs workspace: kblas_posv_vbatch_wsquery.
  * A non-positive n or an out-of-range lda/ldb gives info = -(argument index). */
