@@ -73,7 +73,7 @@ __device__ __forceinline__ void tri_ld4(const T *p, T (&m)[4]) {
 // four FP64 FMAs keep the pipe busy for 256 cycles, so nothing else of a row
 // costs time but the one addition that joins its two sums. Against a row at a
 // time with four partial sums (20,000 triangles of order 64 on 64 vectors, copies
-// of the operands included): TRSM 6450 -> 5810 us, TRMM 6660 -> 6110 us; the FP64
+// of the operands included): TRSM 6450 -> 5666 us, TRMM 6665 -> 5744 us; the FP64
 // pipe needs 4570.
 template <typename T>
 __device__ __forceinline__ void tri_rows4(const T *g, const T *x, int i0, T (&s)[4]) {
@@ -95,21 +95,49 @@ __device__ __forceinline__ void tri_rows4(const T *g, const T *x, int i0, T (&s)
   for (int u = 0; u < 4; u++) s[u] = e[u] + o[u];
 }
 
-// One vector against a triangle that is read from global memory.
-template <typename T, int OP, class M>
-__device__ __forceinline__ void tri_direct(T *x, const T *sD, int K, T alpha, const M &Mval) {
-  if (OP == 0) {
-    for (int i = 0; i < K; i++) {
-      T s = x[i];
-      for (int k = 0; k < i; k++) s -= Mval(i, k) * x[k];
-      x[i] = s * sD[i];
+// The same sum for one row: the last rows when their number is no multiple of four
+// (the FMAs of rows that are not there would cost as much as others: 40% of them at
+// order 9).
+template <typename T>
+__device__ __forceinline__ T tri_row1(const T *g, const T *x, int n) {
+  T e = T(0), o = T(0);
+  int k = 0;
+#pragma unroll 2
+  for (; k + 1 < n; k += 2) {
+    e += g[4 * k] * x[k];
+    o += g[4 * k + 4] * x[k + 1];
+  }
+  if (k < n) e += g[4 * k] * x[k];
+  return e + o;
+}
+
+// One vector against a triangle that is read from global memory: M(i, k) at
+// M[i si + k sk]. One sum per row, eight products' loads ahead of their FMAs: with
+// few warps on an SM (the vectors of such orders take its shared memory) the loads'
+// latency counts. us without / with it, 500 FP64 triangles of order 150 on 150
+// vectors: TRSM 4925 / 3864, TRMM 3904 / 3712; 3,000 FP32 ones of order 190 on 12:
+// TRSM 733 / 658, TRMM 632 / 615.
+template <typename T, int OP>
+__device__ __forceinline__ void tri_direct(T *x, const T *sD, int K, T alpha, const T *M, ptrdiff_t si,
+                                           ptrdiff_t sk) {
+  for (int r = 0; r < K; r++) {
+    const int i = OP == 0 ? r : K - 1 - r;
+    const T *p = M + i * si;
+    T s = OP == 0 ? x[i] : sD[i] * x[i];
+    int k = 0;
+    for (; k + 8 <= i; k += 8) {
+      T m[8], y[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        m[u] = p[u * sk];
+        y[u] = x[k + u];
+      }
+      p += 8 * sk;
+#pragma unroll
+      for (int u = 0; u < 8; u++) s += OP == 0 ? -m[u] * y[u] : m[u] * y[u];
     }
-  } else {
-    for (int i = K - 1; i >= 0; i--) {
-      T s = sD[i] * x[i];
-      for (int k = 0; k < i; k++) s += Mval(i, k) * x[k];
-      x[i] = alpha * s;
-    }
+    for (; k < i; k++, p += sk) s += OP == 0 ? -*p * x[k] : *p * x[k];
+    x[i] = OP == 0 ? s * sD[i] : alpha * s;
   }
 }
 
@@ -185,40 +213,45 @@ __global__ void tri_vec_kernel(TriDesc d, T alpha, AccA A, AccB B, Dims dims, lo
     if (tid < vc) {
       T *x = sX + (size_t)tid * d.ldx;
       if (!d.staged) {
-        tri_direct<T, OP>(x, sD, K, alpha, Mval);
+        const ptrdiff_t down = d.rev ? -1 : 1;
+        tri_direct<T, OP>(x, sD, K, alpha, d.rev ? Ag + (size_t)(K - 1) * (lda + 1) : Ag,
+                          d.mtrans ? down * lda : down, d.mtrans ? down : down * lda);
       } else if (OP == 0) {
-        for (int i0 = 0; i0 < K; i0 += 4) {
+        int i0 = 0;
+        for (; i0 + 4 <= K; i0 += 4) {
           T s[4];
-          tri_rows4(sM + tri_row4(i0 >> 2), x, i0, s);
+          if (i0 > 0) tri_rows4(sM + tri_row4(i0 >> 2), x, i0, s);
           const T *tr = sM + tri_row4(i0 >> 2) + 4 * i0;  // (row, i0 + v) at tr[4 v + row - i0]
 #pragma unroll
           for (int u = 0; u < 4; u++) {
-            if (i0 + u < K) {
-              T v = x[i0 + u] - s[u];
+            T v = i0 > 0 ? x[i0 + u] - s[u] : x[i0 + u];
 #pragma unroll
-              for (int q = 0; q < u; q++) v -= tr[4 * q + u] * s[q];
-              s[u] = v * sD[i0 + u];  // solved
-              x[i0 + u] = s[u];
-            }
+            for (int q = 0; q < u; q++) v -= tr[4 * q + u] * s[q];
+            s[u] = v * sD[i0 + u];  // solved
+            x[i0 + u] = s[u];
           }
         }
+        for (int i = i0; i < K; i++)
+          x[i] = (x[i] - tri_row1(sM + tri_row4(i0 >> 2) + (i - i0), x, i)) * sD[i];
       } else {
-        for (int i0 = (K - 1) & ~3; i0 >= 0; i0 -= 4) {
+        const int full = K & ~3;
+        for (int i = K - 1; i >= full; i--) {
+          const T s = tri_row1(sM + tri_row4(full >> 2) + (i - full), x, i) + sD[i] * x[i];
+          x[i] = alpha == T(1) ? s : alpha * s;
+        }
+        for (int i0 = full - 4; i0 >= 0; i0 -= 4) {
           T s[4], xi[4];
           tri_rows4(sM + tri_row4(i0 >> 2), x, i0, s);
           const T *tr = sM + tri_row4(i0 >> 2) + 4 * i0;
 #pragma unroll
           for (int u = 0; u < 4; u++) {
-            if (i0 + u < K) {
-              xi[u] = x[i0 + u];
+            xi[u] = x[i0 + u];
 #pragma unroll
-              for (int q = 0; q < u; q++) s[u] += tr[4 * q + u] * xi[q];
-              s[u] += sD[i0 + u] * xi[u];
-            }
+            for (int q = 0; q < u; q++) s[u] += tr[4 * q + u] * xi[q];
+            s[u] += sD[i0 + u] * xi[u];
           }
 #pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (i0 + u < K) x[i0 + u] = alpha == T(1) ? s[u] : alpha * s[u];
+          for (int u = 0; u < 4; u++) x[i0 + u] = alpha == T(1) ? s[u] : alpha * s[u];
         }
       }
     }
@@ -251,7 +284,7 @@ static int plan_tri(KBlasHandle *h, char side, char uplo, char trans, char diag,
   d.ldx = Kmax | 1;
   const int limit = max_smem(h);
   const size_t tri_bytes = (size_t)tri_row4((Kmax + 3) >> 2) * sizeof(T);
-  d.staged = tri_bytes <= 64 * 1024;
+  d.staged = (size_t)Kmax * (Kmax + 1) / 2 * sizeof(T) <= 64 * 1024;
   int VC = Vmax < 64 ? Vmax : 64;
   if (VC < 1) VC = 1;
   auto bytes = [&](int vc, bool st) {
