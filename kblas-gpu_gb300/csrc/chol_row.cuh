@@ -7,6 +7,10 @@
 // warp). Bound by shared-memory loads: per column k a warp loads the 8 pivot
 // rows' entries as two 128-bit broadcasts (8 cycles of the load pipe) and its own
 // R entries for 8 R FMAs, hence up to four rows a lane.
+//
+// Every warp reads the 8 pivot rows of the block from A, so with several warps no
+// thread writes them to A before the block's barrier; every other row is read and
+// written by one lane only.
 #pragma once
 
 #include "chol_fix.cuh"
@@ -35,7 +39,8 @@ __device__ __forceinline__ void row_ld8(const float *p, float (&y)[FX_W]) {
 }
 
 // The columns C..C+7 of R rows a lane; returns the failing column (1-based, the
-// same in every warp) or 0. Finished columns go to Xs and to A.
+// same in every warp) or 0. Finished columns go to Xs and to A, the pivot rows (with
+// several warps) to Xs alone: row_store_pivots.
 template <int NW, int R>
 __device__ __forceinline__ int row_block(const FixLayout &F, float *A, int lda, float *Xs, int C,
                                          float *rinv, float *yd)
@@ -99,7 +104,7 @@ __device__ __forceinline__ int row_block(const FixLayout &F, float *A, int lda, 
         x[r] = (r == 0 && lane == c) ? s : a[r][c] * q;
         if (own[r] && row[r] >= C + c) {
           col[row[r]] = x[r];
-          A[(size_t)row[r] + (size_t)(C + c) * lda] = x[r];
+          if (NW == 1 || r > 0 || lane >= FX_W) A[(size_t)row[r] + (size_t)(C + c) * lda] = x[r];
         }
       }
       col += ld;
@@ -116,6 +121,17 @@ __device__ __forceinline__ int row_block(const FixLayout &F, float *A, int lda, 
     }
   }
   return 0;
+}
+
+// The pivot rows of the block of columns C..C+7 from Xs to A, the columns before the
+// failing one (fail, 1-based, or 0): by the lanes that put them into Xs, after the
+// barrier that ends every warp's reading of them.
+__device__ __forceinline__ void row_store_pivots(const FixLayout &F, float *A, int lda, const float *Xs,
+                                                 int C, int fail)
+{
+  const int i = C + (int)threadIdx.x, end = min(fail ? fail - 1 : F.n, C + FX_W);
+  if (threadIdx.x < FX_W && i < F.n)
+    for (int k = C; k < end && k <= i; k++) A[(size_t)i + (size_t)k * lda] = Xs[F.col(k) + i];
 }
 
 // MODE as in chol_kernels.cuh.
@@ -148,6 +164,7 @@ chol_row_kernel(int n, int m, AccA A, int lda, AccB B, int ldb, int *info)
       }
       if (NW == 1) __syncwarp();
       else if (__syncthreads_or(fail) && !fail) fail = n + 1;  // (its value is warp 0's to report)
+      if (NW > 1) row_store_pivots(F, Ag, lda, Xs, C, fail);
     }
     if (threadIdx.x == 0 && info) info[b] = fail;
     if (fail) return;
