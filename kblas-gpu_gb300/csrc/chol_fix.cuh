@@ -1,36 +1,53 @@
 // chol_fix.cuh -- FP64 Cholesky in 64-bit fixed point on the integer pipe, and
 // the FP64 triangular solves with its factor (panel path, n > 32).
 //
-// Why: the part retires 2 FP64 FMA lanes per clock and SM, but 30 lanes of a 32 x
-// 32 -> 64-bit integer multiply-add and 64 or more of an FP32 FMA, and one of the
-// former with two of the latter make a product of two 56-bit numbers. A Cholesky
-// factor suits fixed point: row i of L is bounded by sqrt(a_ii), so its scale
-// 2^E_i > sqrt(a_ii) is known beforehand.
+// Why: the part retires 2 FP64 FMA lanes per clock and SM but about 30 lanes of
+// a 32 x 32 -> 64-bit integer multiply-add, and three of those make a product
+// of two 60-bit numbers. A Cholesky factor suits fixed point: row i of L is
+// bounded by sqrt(a_ii), so its scale 2^E_i > sqrt(a_ii) is known beforehand.
 //
-//   L(i, k) = X 2^(E_i - 56),  X = h 2^25 + l, |X| < 2^56, l in [-2^24, 2^24)
+//   L(i, k) = X 2^(E_i - 59),  X = hi 2^30 + lo, |X| < 2^59, lo in [-2^29, 2^29)
 //   S(i, j) = a_ij - sum_k L(i, k) L(j, k) in units of 2^(E_i + E_j - 62)
 //
-// The products h h' are summed exactly in 64 bits: sum |h|^2 of a row is below
-// 2^62 (Cauchy-Schwarz). The products h l' + l h', 2^-32 of the scales, are summed
-// in FP32 (l is exact in FP32, h rounded to 24 bits) and join the 64-bit sum every
-// FX_FOLD = 16 columns, so that their roundings stay 2^-24 of 2^-31 of the scales;
-// l l' is below 2^-64. The pivot's reciprocal square root (FP32 seed, one cubic
-// step) and the scaling of a column are 64-bit integer work. Measured against quad
-// precision on shifted, conditioned and covariance matrices of order 33..400, the
-// errors of L and of the solutions are 0.3..1.0 times those of FP64 FMAs. The
-// backward error |dA_ij| is a few 2^-57 sqrt(K) sqrt(a_ii a_jj) (bound of a chain of
-// FP64 FMAs: K 2^-53 sqrt(a_ii a_jj)).
+// A product adds hi hi' to one 64-bit sum and hi lo' + lo hi' to another (lo lo'
+// is below 2^-60 of the scales). The sums cannot overflow: sum |hi|^2 of a row
+// is at most 2^58 (Cauchy-Schwarz), so |sum hi hi'| <= 2^58 and
+// |sum hi lo' + lo hi'| <= 2 2^29 sqrt(K) 2^29: for K = FX_CARRY = 128 columns,
+// after which the second sum's upper part is carried into the first, <= 2^62.6.
+// The pivot's reciprocal square root (FP32 seed, one cubic step) and the scaling of
+// a column are 64-bit integer work too. The backward error |dA_ij| is a few
+// 2^-60 sqrt(K) sqrt(a_ii a_jj), where a chain of FP64 FMAs has, entry by entry,
+// about 2^-53 (|L| |L^T|)_ij.
+//
+// So an entry far below sqrt(a_ii a_jj) would keep fewer bits than in FP64, and a
+// component of a solution that hangs on such entries alone (the far end of a
+// decaying covariance for a unit right-hand side, weakly coupled unknowns) would
+// be wrong in as many. So these are counted (fx_weak): a coupling of the unknowns
+// i > j is an entry with a_ij or S(i, j) not zero, t the bits by which the larger of
+// both lies below its scale 2^(E_i + E_j), and an unknown whose couplings have
+// max(0, t - 8) at more than 1 in the mean leaves the matrix to the FP64 path.
+// (Single small entries among others of the same unknowns, as random matrices have
+// them, do not matter: the others' rounding reaches every component that theirs
+// reaches.) Against quad precision, FP64 FMAs / fixed point, on the matrices that
+// stay: root mean square of |A - L L^T|_ij / (|L| |L^T|)_ij in 2^-53, G G^T + n I of
+// order 128 1.2 / 1.0, condition 1e6 of order 64 0.5 / 0.4, squared-exponential
+// covariance of length 0.3 and order 160 0.35 / 0.41; the largest relative error of a
+// component of A^-1 e_1 7e-14 / 4e-13, 4e-10 / 5e-11 and 1.8e-9 / 1.5e-9. The same
+// covariance with length 0.05, taken in fixed point: 3e-11 / 3e-6. 56-bit entries with
+// the cross products summed in FP32 are faster (10,000 POSV of order 64, four right-hand
+// sides 968 us against 1139, 2,000 of order 150 1944 against 2405), but not as accurate
+// as FP64 FMAs entry by entry: 1.2 / 4.8 on the shifted matrices.
 //
 // A matrix that does not fit the scheme -- a pivot below 2^-42 a_jj, an entry
 // or a row of L above its bound (only when A is not positive definite), an
-// infinity or NaN, a diagonal outside 2^+-800 -- is left to the FP64 path,
-// which starts again from A (nothing has been written), so info and the
-// columns before a failing pivot are that path's.
+// infinity or NaN, a diagonal outside 2^+-800, weak couplings -- is left to the
+// FP64 path, which starts again from A (nothing has been written), so info and
+// the columns before a failing pivot are that path's.
 //
 // Work split: left-looking by blocks of 8 columns, one matrix row per lane (or
 // two): a lane keeps the 8 pairs of sums of each of its rows, loads its own
 // X(i, k) (8 bytes, lanes consecutive) and the 8 pivot rows' X(C + c, k) as four
-// 128-bit broadcasts: 24 (48) products for 5 (6) loads. Lanes 0..7 of every
+// 128-bit broadcasts: 24 (48) multiply-adds for 5 (6) loads. Lanes 0..7 of every
 // warp hold the block's 8 pivot rows, so each warp finds the pivots by itself:
 // the chain of 8 pivots, which the other warps would have to wait for, costs
 // every warp 8 lanes instead, and a block needs one barrier.
@@ -42,7 +59,7 @@
 namespace kgb {
 
 constexpr int FX_W = 8;         // columns per block
-constexpr int FX_FOLD = 16;     // columns after which the FP32 sums are folded
+constexpr int FX_CARRY = 128;   // columns after which the sums of cross products are carried
 constexpr int FX_DMIN_LOG = 20; // smallest pivot taken, in units of 2^(2 E - 62)
 
 // The lower triangle in blocks of 8 columns: block b holds the rows 8 b .. of
@@ -81,21 +98,27 @@ __device__ __forceinline__ int fx_scale(double a, int &bad) {
   return ((((hi + 0x100) >> 20) - 1023) >> 1) + 1;
 }
 
-// a 2^(62 - es), cut towards zero; bad if |a| >= 2^es (infinities and NaNs too)
+// a 2^(62 - es), cut towards zero (but 1 at least, unless a is zero); bad if
+// |a| >= 2^es (infinities and NaNs too)
 __device__ __forceinline__ long long fx_from(double a, int es, int &bad) {
   const uint32_t hi = (uint32_t)__double2hiint(a), lo = (uint32_t)__double2loint(a);
   const int r = es + 1022 - (int)((hi >> 20) & 0x7ffu);
   if (r < 0) bad = 1;
-  const long long m =
+  long long m =
       (long long)(((((unsigned long long)((hi & 0xfffffu) | 0x100000u)) << 32) | lo) << 9 >> min(max(r, 0), 63));
+  if (m == 0) m = (hi << 1 | lo) != 0;
   const long long s = (long long)((int)hi >> 31);
   return (m ^ s) - s;
 }
 
-// The FP32 sum of h l' + l h' (units of 2^25 of those of S) joins hh.
-__device__ __forceinline__ void fx_fold(long long &hh, float &lo) {
-  hh += (long long)__float2int_rn(lo * 1.862645149230957e-9f) * 16;  // 2^-29
-  lo = 0.f;
+// The two sums of products, in units of S.
+__device__ __forceinline__ long long fx_sum(long long hh, long long mid) {
+  return (long long)((unsigned long long)hh << 4) + ((mid + (1ll << 25)) >> 26);
+}
+// Moves what it can of the cross products to the sum of hi hi', without rounding.
+__device__ __forceinline__ void fx_carry(long long &hh, long long &mid) {
+  hh += mid >> 30;
+  mid &= (1ll << 30) - 1;
 }
 
 // Reciprocal square root of a pivot: rho = rh 2^31 + rl = 2^92 / sqrt(d 4^z), z
@@ -105,7 +128,7 @@ struct FixPivot {
 };
 // Pivots and the pivot rows of the block at hand, one copy per warp.
 struct FixScratch {
-  double yd[FX_W][FX_W];  // [column][row]
+  double yd[FX_W][FX_W];  // limbs, [column][row]
   FixPivot pv[FX_W];
 };
 
@@ -135,7 +158,7 @@ __device__ __forceinline__ FixPivot fx_rsqrt(long long d) {
   return p;
 }
 
-// s rho 2^(z - 67): the entry of L in units of 2^(E - 56). bad gets set bits if s
+// s rho 2^(z - 64): the entry of L in units of 2^(E - 59). bad gets set bits if s
 // or the entry is out of range (the row's squares then exceed a_ii).
 __device__ __forceinline__ long long fx_scale_entry(long long s, const FixPivot &p, unsigned &bad) {
   const int sh = (int)(s >> 32);
@@ -144,41 +167,39 @@ __device__ __forceinline__ long long fx_scale_entry(long long s, const FixPivot 
   const int th = (int)(t >> 31), tl = (int)t & 0x7fffffff;
   long long m = (long long)th * p.rl;
   m += (long long)tl * p.rh;
-  long long x = (m >> 31) + 16;
+  long long x = (m >> 31) + 2;
   x += (long long)th * p.rh;
-  x >>= 5;
+  x >>= 2;
   const int xh = (int)(x >> 32);
-  bad |= (unsigned)(xh ^ (xh >> 31)) >> 24;
+  bad |= (unsigned)(xh ^ (xh >> 31)) >> 27;
   return x;
 }
 
-// h and l (as FP32) as the words of a double (never used as a floating-point
-// value).
+// Both limbs as the words of a double (never used as a floating-point value).
 __device__ __forceinline__ double fx_pack(long long x) {
-  const int l = (int)((unsigned)x << 7) >> 7;
-  return __hiloint2double((int)((x - l) >> 25), __float_as_int((float)l));
+  const int lo = (int)((unsigned)x << 2) >> 2;
+  return __hiloint2double((int)((x - lo) >> 30), lo);
 }
-__device__ __forceinline__ float fx_l(double v) { return __int_as_float(__double2loint(v)); }
 __device__ __forceinline__ long long fx_unpack(double v) {
-  return ((long long)__double2hiint(v) << 25) + __float2int_rn(fx_l(v));
+  return ((long long)__double2hiint(v) << 30) + __double2loint(v);
 }
 
-// The 8 products of x with y[c0..7]; yf: FP32 of y's h.
-__device__ __forceinline__ void fx_mac(long long (&hh)[FX_W], float (&lo)[FX_W], double x,
-                                       const double (&y)[FX_W], const float (&yf)[FX_W], int c0) {
-  const int xh = __double2hiint(x);
-  const float xf = (float)xh, xl = fx_l(x);
+// The 8 products of x with y[c0..7], each kind of product in turn: the two that
+// share a sum are then 8 instructions apart.
+__device__ __forceinline__ void fx_mac(long long (&hh)[FX_W], long long (&mid)[FX_W], double x,
+                                       const double (&y)[FX_W], int c0) {
+  const int xh = __double2hiint(x), xl = __double2loint(x);
 #pragma unroll
   for (int c = 0; c < FX_W; c++)
-    if (c >= c0) {
-      hh[c] += (long long)xh * __double2hiint(y[c]);
-      lo[c] = fmaf(xf, fx_l(y[c]), lo[c]);
-    }
+    if (c >= c0) hh[c] += (long long)xh * __double2hiint(y[c]);
 #pragma unroll
   for (int c = 0; c < FX_W; c++)
-    if (c >= c0) lo[c] = fmaf(xl, yf[c], lo[c]);
+    if (c >= c0) mid[c] += (long long)xh * __double2loint(y[c]);
+#pragma unroll
+  for (int c = 0; c < FX_W; c++)
+    if (c >= c0) mid[c] += (long long)xl * __double2hiint(y[c]);
 }
-// 8 consecutive elements, 16-byte aligned
+// 8 consecutive limbs, 16-byte aligned
 __device__ __forceinline__ void fx_ld8(const double *p, double (&y)[FX_W]) {
 #pragma unroll
   for (int c = 0; c < FX_W; c += 2) {
@@ -187,10 +208,17 @@ __device__ __forceinline__ void fx_ld8(const double *p, double (&y)[FX_W]) {
     y[c + 1] = v.y;
   }
 }
-__device__ __forceinline__ void fx_hf(const double (&y)[FX_W], float (&yf)[FX_W], int c0) {
-#pragma unroll
-  for (int c = 0; c < FX_W; c++)
-    if (c >= c0) yf[c] = (float)__double2hiint(y[c]);
+// A coupling's share of its two unknowns' sums, plus 1 (so 1 if there is none): an
+// unknown whose sum of shares ends above zero has couplings that are too weak. Where the line lies: an
+// entry's error is about 2^-59..2^-60 of its scale, which FP64 FMAs reach 6 bits below
+// it, and with 8 bits free and 1 more in the mean all of G G^T + n I up to order 1024
+// (0.0..0.5 in the mean of the worst unknown) and random matrices of condition
+// 1e2..1e8 (0.0..0.2) stay; squared-exponential covariances on the unit square stay
+// from length 0.27 on (at 0.25 1.3..2.2, at 0.2 2.3..5.8).
+__device__ __forceinline__ int fx_weak(long long a, long long s) {
+  const int ah = (int)(a >> 32), sh = (int)(s >> 32);
+  const int z = __clz((ah ^ (ah >> 31)) | (sh ^ (sh >> 31)));  // 2 at the scale
+  return (a | s) == 0 ? 1 : max(z - 10, 0);
 }
 
 // R rows of a thread against the block of columns C..C+7: the sums over the
@@ -198,12 +226,12 @@ __device__ __forceinline__ void fx_hf(const double (&y)[FX_W], float (&yf)[FX_W]
 template <int R>
 __device__ __forceinline__ void fx_dot(const FixLayout &F, const double *Xs, int C,
                                        const int (&row)[R], long long (&hh)[R][FX_W],
-                                       float (&lo)[R][FX_W])
+                                       long long (&mid)[R][FX_W])
 {
 #pragma unroll
   for (int r = 0; r < R; r++)
 #pragma unroll
-    for (int c = 0; c < FX_W; c++) hh[r][c] = 0, lo[r][c] = 0.f;
+    for (int c = 0; c < FX_W; c++) hh[r][c] = mid[r][c] = 0;
   const double *P = Xs;
   int ld = F.n2;
   for (int K = 0; K < C; K += FX_W) {
@@ -212,23 +240,21 @@ __device__ __forceinline__ void fx_dot(const FixLayout &F, const double *Xs, int
 #pragma unroll 4
     for (int k = 0; k < FX_W; k++) {
       double y[FX_W], x[R];
-      float yf[FX_W];
       fx_ld8(yp, y);
-      fx_hf(y, yf, 0);
 #pragma unroll
       for (int r = 0; r < R; r++) x[r] = xp[row[r]];
       yp += ld;
       xp += ld;
 #pragma unroll
-      for (int r = 0; r < R; r++) fx_mac(hh[r], lo[r], x[r], y, yf, 0);
+      for (int r = 0; r < R; r++) fx_mac(hh[r], mid[r], x[r], y, 0);
     }
     P += FX_W * ld;
     ld -= FX_W;
-    if (((K + FX_W) & (FX_FOLD - 1)) == 0) {
+    if (((K + FX_W) & (FX_CARRY - 1)) == 0) {
 #pragma unroll
       for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int c = 0; c < FX_W; c++) fx_fold(hh[r][c], lo[r][c]);
+        for (int c = 0; c < FX_W; c++) fx_carry(hh[r][c], mid[r][c]);
     }
   }
 }
@@ -236,7 +262,9 @@ __device__ __forceinline__ void fx_dot(const FixLayout &F, const double *Xs, int
 // The same with X in global memory: the next 8 columns of the warp's rows and of
 // the pivot rows are copied to shared memory while the current 8 are multiplied,
 // so the latency of L2 is paid once per block, not once per 4 columns (500 systems
-// of order 512: 13.6 -> 11.6 ms).
+// of order 512: 13.6 -> 11.6 ms). A's 8 columns come last, the same way, and into av
+// (zeros right of the diagonal and of the matrix): registers that hold them during the
+// products spill.
 struct FixStage {
   double x[2][FX_W][64];
   double y[2][FX_W][FX_W];
@@ -248,84 +276,99 @@ __device__ __forceinline__ void fx_copy8(double *dst, const double *src) {
                : "memory");
 }
 template <int R>
-__device__ __forceinline__ void fx_dot_staged(const FixLayout &F, const double *Xs, int C,
-                                              const int (&row)[R], long long (&hh)[R][FX_W],
-                                              float (&lo)[R][FX_W], FixStage *st)
+__device__ __forceinline__ void fx_dot_staged(const FixLayout &F, const double *A, int lda,
+                                              const double *Xs, int C, const int (&row)[R],
+                                              const int (&ri)[R], long long (&hh)[R][FX_W],
+                                              long long (&mid)[R][FX_W], double (&av)[R][FX_W],
+                                              FixStage *st)
 {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int r = 0; r < R; r++)
 #pragma unroll
-    for (int c = 0; c < FX_W; c++) hh[r][c] = 0, lo[r][c] = 0.f;
+    for (int c = 0; c < FX_W; c++) hh[r][c] = mid[r][c] = 0;
   const double *P = Xs;  // the block to be copied next
   int ld = F.n2;
   auto copy = [&](int K) {
     const int buf = (K / FX_W) & 1;
+    if (K < C) {
 #pragma unroll
-    for (int c = 0; c < FX_W; c++)
+      for (int c = 0; c < FX_W; c++)
 #pragma unroll
-      for (int r = 0; r < R; r++) fx_copy8(&st->x[buf][c][r * 32 + lane], P + c * ld + (row[r] - K));
+        for (int r = 0; r < R; r++) fx_copy8(&st->x[buf][c][r * 32 + lane], P + c * ld + (ri[r] - K));
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int c = e * 4 + (lane >> 3), j = lane & 7;
-      fx_copy8(&st->y[buf][c][j], P + c * ld + (C - K) + j);
+      for (int e = 0; e < 2; e++) {
+        const int c = e * 4 + (lane >> 3), j = lane & 7;
+        fx_copy8(&st->y[buf][c][j], P + c * ld + (C - K) + j);
+      }
+      P += FX_W * ld;
+      ld -= FX_W;
+    } else {
+#pragma unroll
+      for (int c = 0; c < FX_W; c++)
+#pragma unroll
+        for (int r = 0; r < R; r++)
+          if (row[r] < F.n && C + c <= row[r])
+            fx_copy8(&st->x[buf][c][r * 32 + lane], A + (size_t)row[r] + (size_t)(C + c) * lda);
     }
-    P += FX_W * ld;
-    ld -= FX_W;
-  };
-  if (C > 0) copy(0);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int K = 0; K < C; K += FX_W) {
-    if (K + FX_W < C) copy(K + FX_W);
     asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  copy(0);
+  for (int K = 0; K < C; K += FX_W) {
+    copy(K + FX_W);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
     const int buf = (K / FX_W) & 1;
 #pragma unroll 2
     for (int k = 0; k < FX_W; k++) {
       double y[FX_W];
-      float yf[FX_W];
       fx_ld8(st->y[buf][k], y);
-      fx_hf(y, yf, 0);
 #pragma unroll
-      for (int r = 0; r < R; r++) fx_mac(hh[r], lo[r], st->x[buf][k][r * 32 + lane], y, yf, 0);
+      for (int r = 0; r < R; r++) fx_mac(hh[r], mid[r], st->x[buf][k][r * 32 + lane], y, 0);
     }
     __syncwarp();  // before this buffer is copied to again
-    if (((K + FX_W) & (FX_FOLD - 1)) == 0) {
+    if (((K + FX_W) & (FX_CARRY - 1)) == 0) {
 #pragma unroll
       for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int c = 0; c < FX_W; c++) fx_fold(hh[r][c], lo[r][c]);
+        for (int c = 0; c < FX_W; c++) fx_carry(hh[r][c], mid[r][c]);
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  const int buf = (C / FX_W) & 1;
+#pragma unroll
+  for (int c = 0; c < FX_W; c++)
+#pragma unroll
+    for (int r = 0; r < R; r++)  // (each lane reads what it copied itself)
+      av[r][c] = (row[r] < F.n && C + c <= row[r]) ? st->x[buf][c][r * 32 + lane] : 0.0;
 }
 
 // The columns C..C+7 of R rows, after fx_dot. FIRST: row[0] of lanes 0..7 are the
 // pivot rows; otherwise the pivots are the ones that FIRST left in fs (KEEP). own: rows
-// that this thread stores. qs: the squares of each row's entries. False if a
-// pivot is too small: every warp sees the same pivots. bad gets set bits if a
-// row is out of range.
+// that this thread stores. qs: the squares of each row's entries. wk: the sums of
+// weak couplings, the rows' in wr. False if a pivot is too small: every warp sees the
+// same pivots. bad gets set bits if a row is out of range.
 template <int R, bool FIRST, bool KEEP>
 __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C,
                                            const int (&row)[R], const bool (&own)[R],
                                            int *zs, double *rho_s,
-                                           long long (&hh)[R][FX_W], float (&lo)[R][FX_W],
+                                           long long (&hh)[R][FX_W], long long (&mid)[R][FX_W],
                                            long long (&a)[R][FX_W], FixScratch *fs,
-                                           float (&qs)[R], unsigned &bad)
+                                           float (&qs)[R], int *wk, int (&wr)[R],
+                                           unsigned &bad)
 {
   const int lane = threadIdx.x & 31;
   const int ld = F.ld(C / FX_W);
   double *col = Xs + F.col(C);
+  // the columns' sums of this lane, plus R, a byte each (0..44)
+  unsigned wc[2] = {R * 0x01010101u, R * 0x01010101u};
 #pragma unroll
   for (int c = 0; c < FX_W; c++) {
     if (C + c < F.n) {
       long long s[R];
       FixPivot pv;
 #pragma unroll
-      for (int r = 0; r < R; r++) {
-        fx_fold(hh[r][c], lo[r][c]);
-        s[r] = a[r][c] - hh[r][c];
-      }
+      for (int r = 0; r < R; r++) s[r] = a[r][c] - fx_sum(hh[r][c], mid[r][c]);
       if (FIRST) {
         const long long d = __shfl_sync(0xffffffffu, s[0], c);
         if (d < (1ll << FX_DMIN_LOG) || d >= (1ll << 62)) return false;
@@ -347,6 +390,11 @@ __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C
           col[row[r]] = x[r];
           const float f = (float)__double2hiint(x[r]);
           qs[r] += f * f;
+          if (row[r] > C + c) {
+            const int w = fx_weak(a[r][c], s[r]) - 1;
+            wr[r] += w;
+            wc[c >> 2] += (unsigned)w << (8 * (c & 3));
+          }
         }
       }
       col += ld;
@@ -356,13 +404,20 @@ __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C
         __syncwarp();
       }
       double y[FX_W];
-      float yf[FX_W];
       fx_ld8(fs->yd[c], y);
-      fx_hf(y, yf, c + 1);
 #pragma unroll
-      for (int r = 0; r < R; r++) fx_mac(hh[r], lo[r], x[r], y, yf, c + 1);
+      for (int r = 0; r < R; r++) fx_mac(hh[r], mid[r], x[r], y, c + 1);
     }
   }
+  // lane c adds up column c's: two columns to a word
+  unsigned mine = 0;
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const unsigned t = __reduce_add_sync(0xffffffffu, (wc[e >> 1] >> (8 * (e & 1))) & 0x00ff00ffu);
+    // columns 4 (e / 2) + e % 2 and two further
+    if ((lane & ~2) == (e >> 1) * 4 + (e & 1)) mine = (lane & 2) ? t >> 16 : t & 0xffffu;
+  }
+  if (lane < FX_W && C + lane < F.n) atomicAdd(wk + C + lane, (int)mine - 32 * R);
   return true;
 }
 
@@ -370,22 +425,16 @@ __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C
 template <int R, bool FIRST, bool BIG>
 __device__ __forceinline__ bool fx_rows(const FixLayout &F, const double *A, int lda, double *Xs,
                                         int C, const int (&row)[R], const bool (&own)[R],
-                                        const int *Es, float *q, int *zs, double *rho_s,
-                                        FixScratch *fs, FixStage *st, unsigned &bad)
+                                        const int *Es, float *q, int *wk, int *zs,
+                                        double *rho_s, FixScratch *fs, FixStage *st,
+                                        unsigned &bad)
 {
   int ri[R];
-  long long a[R][FX_W], hh[R][FX_W];
-  float lo[R][FX_W];
-  {
-    double av[R][FX_W];
+  long long a[R][FX_W], hh[R][FX_W], mid[R][FX_W];
+#pragma unroll
+  for (int r = 0; r < R; r++) ri[r] = min(row[r], F.n - 1);
+  auto fixed = [&](const double (&av)[R][FX_W]) {
     int b = 0;
-#pragma unroll
-    for (int r = 0; r < R; r++) ri[r] = min(row[r], F.n - 1);
-#pragma unroll
-    for (int c = 0; c < FX_W; c++)
-#pragma unroll
-      for (int r = 0; r < R; r++)
-        av[r][c] = (row[r] < F.n && C + c <= row[r]) ? A[(size_t)ri[r] + (size_t)(C + c) * lda] : 0.0;
 #pragma unroll
     for (int c = 0; c < FX_W; c++) {
       const int Ec = Es[min(C + c, F.n - 1)];
@@ -393,20 +442,34 @@ __device__ __forceinline__ bool fx_rows(const FixLayout &F, const double *A, int
       for (int r = 0; r < R; r++) a[r][c] = fx_from(av[r][c], Es[ri[r]] + Ec, b);
     }
     bad |= (unsigned)b;
-  }
-  if (BIG) fx_dot_staged<R>(F, Xs, C, ri, hh, lo, st);
-  else fx_dot<R>(F, Xs, C, ri, hh, lo);
-  float qs[R];
+  };
+  double av[R][FX_W];
+  if (BIG) {
+    fx_dot_staged<R>(F, A, lda, Xs, C, row, ri, hh, mid, av, st);
+    fixed(av);
+  } else {
 #pragma unroll
-  for (int r = 0; r < R; r++) qs[r] = 0.f;
-  const bool ok = fx_columns<R, FIRST, BIG>(F, Xs, C, row, own, zs, rho_s, hh, lo, a, fs, qs, bad);
+    for (int c = 0; c < FX_W; c++)
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        av[r][c] = (row[r] < F.n && C + c <= row[r]) ? A[(size_t)ri[r] + (size_t)(C + c) * lda] : 0.0;
+    fixed(av);
+    fx_dot<R>(F, Xs, C, ri, hh, mid);
+  }
+  float qs[R];
+  int wr[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) qs[r] = 0.f, wr[r] = 0;
+  const bool ok =
+      fx_columns<R, FIRST, BIG>(F, Xs, C, row, own, zs, rho_s, hh, mid, a, fs, qs, wk, wr, bad);
   // a row whose squares add up to more than a_ii: A is not positive definite
 #pragma unroll
   for (int r = 0; r < R; r++)
     if (own[r]) {
       const float v = q[row[r]] + qs[r];
       q[row[r]] = v;
-      if (!(v < 4611686018427387904.0f)) bad = 1;  // 2^62
+      if (!(v < 288230376151711744.0f)) bad = 1;  // 2^58
+      atomicAdd(wk + row[r], wr[r]);
     }
   return ok;
 }
@@ -416,8 +479,9 @@ __device__ __forceinline__ bool fx_rows(const FixLayout &F, const double *A, int
 // what is left (BIG, whose X is in global memory) in turns of 64 rows a warp.
 template <int NW, int R, bool BIG>
 __device__ __forceinline__ bool fx_block(const FixLayout &F, const double *A, int lda, double *Xs,
-                                         int C, const int *Es, float *q, int *zs, double *rho_s,
-                                         FixScratch *fs, FixStage *st, unsigned &bad)
+                                         int C, const int *Es, float *q, int *wk, int *zs,
+                                         double *rho_s, FixScratch *fs, FixStage *st,
+                                         unsigned &bad)
 {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int row[R];
@@ -432,7 +496,7 @@ __device__ __forceinline__ bool fx_block(const FixLayout &F, const double *A, in
   // the pivots at the barrier
   bool ok = true;
   if (w == 0 || C + w * (32 - FX_W) + FX_W < F.n)
-    ok = fx_rows<R, true, BIG>(F, A, lda, Xs, C, row, own, Es, q, zs, rho_s, fs, st, bad);
+    ok = fx_rows<R, true, BIG>(F, A, lda, Xs, C, row, own, Es, q, wk, zs, rho_s, fs, st, bad);
   if (BIG && R == 2) {
     for (int g = C + FX_W + NW * (64 - FX_W); ok && g < F.n; g += NW * 64) {
 #pragma unroll
@@ -440,27 +504,30 @@ __device__ __forceinline__ bool fx_block(const FixLayout &F, const double *A, in
         row[r] = g + (w * R + r) * 32 + lane;
         own[r] = row[r] < F.n;
       }
-      fx_rows<R, false, BIG>(F, A, lda, Xs, C, row, own, Es, q, zs, rho_s, fs, st, bad);
+      fx_rows<R, false, BIG>(F, A, lda, Xs, C, row, own, Es, q, wk, zs, rho_s, fs, st, bad);
     }
   }
   if (NW == 1) __syncwarp();
   else ok = __syncthreads_and(ok);
-  return ok;
+  // the sums of this block's unknowns are complete and stay as they are
+  const int i = C + (lane & (FX_W - 1));
+  return ok && !__any_sync(0xffffffffu, i < F.n && wk[i] > 0);
 }
 
-// Cholesky factor of the lower triangle of A into Xs, by a CTA of NW
+// Cholesky factor of the lower triangle of A into Xs (limbs), by a CTA of NW
 // warps (n <= 8 + 56 NW, or BIG); rho_s, zs: the reciprocal roots of the pivots.
-// Es: n ints, q: n floats. False: the FP64 path has to take the matrix.
+// Es, wk: n ints, q: n floats. False: the FP64 path has to take the matrix.
 // RMAX = 1: n <= 8 + 24 NW.
 template <int NW, bool BIG, int RMAX = 2>
 __device__ __forceinline__ bool fx_potrf(const FixLayout &F, const double *A, int lda, double *Xs,
-                                         int *Es, float *q, int *zs, double *rho_s,
+                                         int *Es, float *q, int *wk, int *zs, double *rho_s,
                                          FixScratch *fs, FixStage *st = nullptr)
 {
   int b = 0;
   for (int i = threadIdx.x; i < F.n; i += 32 * NW) {
     Es[i] = fx_scale(A[(size_t)i + (size_t)i * lda], b);
     q[i] = 0.f;
+    wk[i] = 0;
   }
   if (NW == 1) b = __any_sync(0xffffffffu, b);
   else b = __syncthreads_or(b);
@@ -471,9 +538,9 @@ __device__ __forceinline__ bool fx_potrf(const FixLayout &F, const double *A, in
   int C = 0;
   if (RMAX > 1)
     for (; ok && F.n - C > FX_W + NW * (32 - FX_W); C += FX_W)
-      ok = fx_block<NW, 2, BIG>(F, A, lda, Xs, C, Es, q, zs, rho_s, fs, st, bad);
+      ok = fx_block<NW, 2, BIG>(F, A, lda, Xs, C, Es, q, wk, zs, rho_s, fs, st, bad);
   for (; ok && C < F.n; C += FX_W)
-    ok = fx_block<NW, 1, BIG>(F, A, lda, Xs, C, Es, q, zs, rho_s, fs, st, bad);
+    ok = fx_block<NW, 1, BIG>(F, A, lda, Xs, C, Es, q, wk, zs, rho_s, fs, st, bad);
   // (ok is the same in every warp)
   if (NW == 1) return ok && !__any_sync(0xffffffffu, bad != 0);
   return !__syncthreads_or(!ok || bad != 0);
@@ -509,7 +576,7 @@ __device__ __forceinline__ int fx_potrf_fp64(const FixLayout &F, double *A, int 
   return 0;
 }
 
-// X -> FP64, into A's lower triangle and (keep) in place; the reciprocals of
+// Limbs -> FP64, into A's lower triangle and (keep) in place; the reciprocals of
 // the diagonal replace rho.
 template <int NW>
 __device__ __forceinline__ void fx_store(const FixLayout &F, double *Xs, const int *Es,
@@ -521,7 +588,7 @@ __device__ __forceinline__ void fx_store(const FixLayout &F, double *Xs, const i
   double *P = Xs;
   for (int C = 0; C < F.n; C += FX_W, P += FX_W * ld, ld -= FX_W) {
     for (int i = C + threadIdx.x; i < F.n; i += 32 * NW) {
-      const int e = Es[i] - 56;
+      const int e = Es[i] - 59;
       double *dst = A + (size_t)i + (size_t)C * lda, *src = P + (i - C);
       double v[FX_W];
       // (all loads before any store: the columns right of the diagonal, or of

@@ -26,7 +26,7 @@ struct FixArgs {
 template <int NW, bool FAC_SMEM>
 __host__ __device__ __forceinline__ size_t fix_smem_bytes(int n) {
   const size_t b = (FAC_SMEM ? (size_t)make_fix_layout(n).total() * 8 : NW * sizeof(FixStage)) +
-                   NW * sizeof(FixScratch) + (size_t)n * 20;
+                   NW * sizeof(FixScratch) + (size_t)n * 24;
   return (b + 15) / 16 * 16;
 }
 
@@ -97,11 +97,12 @@ fix_posv_kernel(SysArgs sys, FixArgs fa)
     double *rinv = reinterpret_cast<double *>(p);
     int *Es = reinterpret_cast<int *>(rinv + n), *zs = Es + n;
     float *qs = reinterpret_cast<float *>(zs + n);
+    int *wk = reinterpret_cast<int *>(qs + n);
     bool ok = true;
     if (sys.op == 2) {
       fx_load<NW>(F, A, lda, Xs, rinv);
     } else {
-      ok = fx_potrf<NW, !FAC_SMEM>(F, A, lda, Xs, Es, qs, zs, rinv, fs, st);
+      ok = fx_potrf<NW, !FAC_SMEM>(F, A, lda, Xs, Es, qs, wk, zs, rinv, fs, st);
       if (ok) fx_store<NW>(F, Xs, Es, zs, rinv, A, lda, m > 0);
       if (threadIdx.x == 0) {
         if (ok) {
@@ -138,10 +139,11 @@ fix_small_kernel(int n, int m, AccA Aa, int lda, AccB Ba, int ldb, int *info)
   double *rinv = reinterpret_cast<double *>(fs + 1);
   int *Es = reinterpret_cast<int *>(rinv + n), *zs = Es + n;
   float *qs = reinterpret_cast<float *>(zs + n);
+  int *wk = reinterpret_cast<int *>(qs + n);
   const long long b = blockIdx.x;
   double *A = Aa.get(b);
   int fail = 0;
-  if (fx_potrf<1, false, 1>(F, A, lda, Xs, Es, qs, zs, rinv, fs))
+  if (fx_potrf<1, false, 1>(F, A, lda, Xs, Es, qs, wk, zs, rinv, fs))
     fx_store<1>(F, Xs, Es, zs, rinv, A, lda, MODE == MODE_POSV);
   else
     fail = fx_potrf_fp64(F, A, lda, Xs, rinv);

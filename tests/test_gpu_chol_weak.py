@@ -6,7 +6,8 @@ elsewhere). Bars for the factor and the solutions of weakly coupled unknowns, th
 an FP64 Cholesky factorization (u = 2^-53; the reciprocal pivots' roundings are in the
 added constant):
   |A - L L^T| <= (n + 8) u |L| |L^T|                       entry by entry,
-  |x - X|     <= (3 n + 16) u |A^-1| |L| |L^T| |X| (1 + 1/8) component by component.
+  |x - X|     <= (3 n + 16) u |A^-1| |L| |L^T| |X| (1 + 1/8) component by component,
+and the smallest normal number, 2^-1022: components below it have no FP64 value.
 A matrix that stays in fixed point has in addition, from entries rounded to 2^-60 of
 their rows' scales 2^E <= 2.01 sqrt(a_ii) and a product of low limbs (2^-60) dropped
 per column, (n + 4 sqrt(n) + 8) 2^-60 2^(E_i + E_j), and its root mean square error
@@ -145,6 +146,7 @@ def test_weak_couplings(gpu, handle, kb, kind, n, form):
             x = solve_ld(R, b[s, :, r])
             got = X[s, :, r].astype(LD)
             bar = (3 * n + 16) * U * 1.125 * mul_ld(inv, mul_ld(scale, np.abs(got)[:, None]))[:, 0]
+            bar = bar + LD(2.0 ** -1022)
             assert (np.abs(x - got) <= bar).all(), (s, r)
 
 
