@@ -11,7 +11,8 @@
 //    holds 32/G matrices. The lower triangle lives in shared memory in packed
 //    column-major form. Right-looking: per column, the team leader computes
 //    the pivot, the team scales the column, then the (n-j-1)(n-j)/2 elements
-//    of the trailing triangle are dealt round-robin to the G lanes.
+//    of the trailing triangle are dealt round-robin to the G lanes. With `left`,
+//    only the matrices marked INFO_LEFT in info.
 //  * chol_blocked_kernel (n > 32): one CTA per matrix, left-looking by panels
 //    of NB columns. Each panel (rows J..n-1) is staged in shared memory,
 //    updated with the already final columns (read from the matrix itself,
@@ -36,6 +37,9 @@ namespace kgb {
 
 enum { MODE_POTRF = 0, MODE_POSV = 1, MODE_POTRS = 2 };
 
+// info of a matrix that a first launch leaves to the next one of the same call.
+constexpr int INFO_LEFT = -1;
+
 // Shared memory bytes of one team (matrix + reciprocals + RHS chunk).
 template <typename T>
 __host__ __device__ __forceinline__ size_t team_smem_elems(int n, int rc) {
@@ -44,7 +48,8 @@ __host__ __device__ __forceinline__ size_t team_smem_elems(int n, int rc) {
 
 template <typename T, int G, int NT, int MODE, class AccA, class AccB>
 __global__ void __launch_bounds__(NT)
-chol_team_kernel(int n, int m, int rc, AccA A, int lda, AccB B, int ldb, long long batch, int *info)
+chol_team_kernel(int n, int m, int rc, AccA A, int lda, AccB B, int ldb, long long batch, int *info,
+                 int left)
 {
   static_assert(32 % G == 0, "team size must divide the warp");
   constexpr int TPB = NT / G;
@@ -52,7 +57,8 @@ chol_team_kernel(int n, int m, int rc, AccA A, int lda, AccB B, int ldb, long lo
   const int team = threadIdx.x / G;
   const int r = threadIdx.x % G;
   const long long b = (long long)blockIdx.x * TPB + team;
-  const bool active = b < batch;
+  const bool active = b < batch && (!left || info[b] == INFO_LEFT);
+  if (left && !__any_sync(0xffffffffu, active)) return;
 
   const size_t per_team = team_smem_elems<T>(n, rc);
   T *sL = reinterpret_cast<T *>(smem_raw) + (size_t)team * per_team;

@@ -126,11 +126,13 @@ fix_posv_kernel(SysArgs sys, FixArgs fa)
 
 // POTRF / POSV of orders up to 32, one warp per system and one row per lane,
 // without workspace: a matrix that does not fit the fixed-point scheme is
-// factored again in FP64 by the same warp. 4 KB to 7 KB of shared memory; 16
+// factored again in FP64 by the same warp or (leave) marked in info, with
+// INFO_LEFT, for chol_team_kernel. 4 KB to 7 KB of shared memory; FIX_SMALL_CTAS
 // CTAs per SM leave 128 registers to a thread.
+constexpr int FIX_SMALL_CTAS = 16;
 template <int MODE, class AccA, class AccB>
-__global__ void __launch_bounds__(32, 16)
-fix_small_kernel(int n, int m, AccA Aa, int lda, AccB Ba, int ldb, int *info)
+__global__ void __launch_bounds__(32, FIX_SMALL_CTAS)
+fix_small_kernel(int n, int m, AccA Aa, int lda, AccB Ba, int ldb, int *info, int leave)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const FixLayout F = make_fix_layout(n);
@@ -145,6 +147,8 @@ fix_small_kernel(int n, int m, AccA Aa, int lda, AccB Ba, int ldb, int *info)
   int fail = 0;
   if (fx_potrf<1, false, 1>(F, A, lda, Xs, Es, qs, wk, zs, rinv, fs))
     fx_store<1>(F, Xs, Es, zs, rinv, A, lda, MODE == MODE_POSV);
+  else if (leave)
+    fail = INFO_LEFT;
   else
     fail = fx_potrf_fp64(F, A, lda, Xs, rinv);
   if (threadIdx.x == 0 && info) info[b] = fail;

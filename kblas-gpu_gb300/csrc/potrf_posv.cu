@@ -5,13 +5,15 @@
 // Xpotrs_batch.cu:87-165 and Xposv_batch.cu:92-178 (same names, arguments,
 // flag support and return codes). Unlike the reference (host recursion over
 // TRSM + SYRK + cuBLAS GEMM, 4 launches at n = 32 and one HBM pass per level),
-// every call is ONE kernel launch: for n <= 32 the team kernel (POTRS of real
-// types: the register kernel, chol_reg.cuh; FP64 POTRF / POSV from order 17: the
-// fixed-point kernel, fix_kernel.cuh) and, above,
-// the fixed-point kernels (double precision, when the workspace the
-// wsqueries request is allocated; what does not fit fixed point goes on to the
-// persistent FP64 panel kernel) or the blocked panel kernel (see
-// chol_kernels.cuh).
+// a call is one kernel launch, or two where the first works in fixed point:
+// for n <= 32 the team kernel (POTRS of real types: the register kernel,
+// chol_reg.cuh; FP64 POTRF / POSV from order 17: the fixed-point kernel,
+// fix_kernel.cuh, which in large batches leaves what does not fit it to the
+// team kernel); above, FP32 the row kernel (chol_row.cuh) as long as the
+// factor fits in shared memory, FP64 the fixed-point kernels (posv_fix.cu, when
+// the workspace the wsqueries request is allocated; a memset comes before them,
+// and what does not fit goes on to the persistent FP64 panel kernel), otherwise
+// the blocked panel kernel (see chol_kernels.cuh).
 #include <stdio.h>
 #include <type_traits>
 
@@ -38,7 +40,7 @@ static inline int team_size_for(int n, bool dbl) {
 
 template <typename T, int G, int MODE, class AccA, class AccB>
 static int launch_team(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int ldb,
-                       long long batch, int *info) {
+                       long long batch, int *info, int left) {
   constexpr int NT = 128;
   constexpr int TPB = NT / G;
   int rc = (MODE == MODE_POTRF) ? 0 : (m < 8 ? m : 8);
@@ -47,7 +49,7 @@ static int launch_team(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, in
   int st = set_smem(kern, smem);
   if (st != KBLAS_Success) return st;
   long long grid = (batch + TPB - 1) / TPB;
-  kern<<<(unsigned)grid, NT, smem, h->stream>>>(n, m, rc, A, lda, B, ldb, batch, info);
+  kern<<<(unsigned)grid, NT, smem, h->stream>>>(n, m, rc, A, lda, B, ldb, batch, info, left);
   KGB_LAUNCH_CHECK("chol_team_kernel");
   return KBLAS_Success;
 }
@@ -83,9 +85,9 @@ static int launch_blocked_nb(KBlasHandle *h, int n, int m, AccA A, int lda, AccB
 
 template <int MODE, class AccA, class AccB>
 static int launch_fix_small(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int ldb,
-                            long long batch, int *info) {
+                            long long batch, int *info, int leave) {
   auto kern = fix_small_kernel<MODE, AccA, AccB>;
-  kern<<<(unsigned)batch, 32, fix_smem_bytes<1, true>(n), h->stream>>>(n, m, A, lda, B, ldb, info);
+  kern<<<(unsigned)batch, 32, fix_smem_bytes<1, true>(n), h->stream>>>(n, m, A, lda, B, ldb, info, leave);
   KGB_LAUNCH_CHECK("fix_small_kernel");
   return KBLAS_Success;
 }
@@ -103,14 +105,26 @@ static int launch_row(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int
   return KBLAS_Success;
 }
 
-// FP64 POTRF / POSV from this order to 32: in fixed point, a warp per system
-// (10,000 POTRF + POTRS of order 32 412 -> 274 us, 200 POSV of order 24 92 -> 33 us,
-// copies of the operands included). Below, half of the warp's lanes would idle.
-constexpr int FIX_SMALL_MIN = 17;
+// FP64 POTRF / POSV of orders FIX_SMALL_MIN..32: in fixed point, a warp per system, as
+// long as the batch is one wave of its warps; from FIX_SMALL_MANY on any batch. us of
+// POSV with one right-hand side, copies of the operands included, chol_team_kernel /
+// fix_small_kernel, for batches of 200, 2,000 and 10,000:
+//   order 12  43 / 25,  47 / 36,  54 / 106     order 24   93 / 36,  93 / 52, 159 / 185
+//   order 16  52 / 29,  52 / 38,  84 / 124     order 28  125 / 45, 127 / 67, 289 / 249
+//   order 17  56 / 31,  58 / 48,  93 / 152     order 32  159 / 46, 163 / 69, 385 / 263
+// (below 17 half of a warp's lanes idle: in batches beyond a wave the team kernel is the
+// faster one by far).
+// Matrices that do not fit fixed point go to FP64 in the same warp within a wave
+// (2,000, all of them: order 24 92 against 93, order 32 134 against 163); in larger
+// batches that warp would be slower than teams of 8 lanes (10,000 of order 32: 648
+// against 385), so these get a second launch, which finds them by the mark in info (421);
+// without an info array to mark them in, large batches stay with the teams.
+constexpr int FIX_SMALL_MIN = 17, FIX_SMALL_MANY = 25;
 
 template <typename T, int MODE, class AccA, class AccB>
 static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, int ldb,
                        long long batch, int *info) {
+  int left = 0;  // the team kernel is to take what fix_small_kernel left
   // POTRS of order <= 32 runs on the register kernel (real types). POTRF and
   // POSV stay on the team kernel: the register factorization keeps a row per
   // lane, so at column c only the rows below c do useful work, and on this
@@ -124,14 +138,22 @@ static int launch_chol(KBlasHandle *h, int n, int m, AccA A, int lda, AccB B, in
     if (n <= 32) return launch_potrs_reg<T, 32>(h, n, m, A, lda, B, ldb, batch);
   }
   if constexpr (MODE != MODE_POTRS && std::is_same<T, double>::value) {
-    if (n >= FIX_SMALL_MIN && n <= 32)
-      return launch_fix_small<MODE>(h, n, m, A, lda, B, ldb, batch, info);
+    if (n >= FIX_SMALL_MIN && n <= 32) {
+      ensure_device_props(h);
+      if (batch <= (long long)h->sm_count * FIX_SMALL_CTAS)
+        return launch_fix_small<MODE>(h, n, m, A, lda, B, ldb, batch, info, 0);
+      if (n >= FIX_SMALL_MANY && info) {
+        int st = launch_fix_small<MODE>(h, n, m, A, lda, B, ldb, batch, info, 1);
+        if (st != KBLAS_Success) return st;
+        left = 1;
+      }
+    }
   }
   if (n <= 32) {
     switch (team_size_for(n, std::is_same<T, double>::value)) {
-      case 2: return launch_team<T, 2, MODE>(h, n, m, A, lda, B, ldb, batch, info);
-      case 4: return launch_team<T, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info);
-      default: return launch_team<T, 8, MODE>(h, n, m, A, lda, B, ldb, batch, info);
+      case 2: return launch_team<T, 2, MODE>(h, n, m, A, lda, B, ldb, batch, info, left);
+      case 4: return launch_team<T, 4, MODE>(h, n, m, A, lda, B, ldb, batch, info, left);
+      default: return launch_team<T, 8, MODE>(h, n, m, A, lda, B, ldb, batch, info, left);
     }
   }
   const int limit = max_smem(h);
