@@ -14,8 +14,9 @@
 // vector while staging. One thread owns one vector (its K elements live in
 // shared memory), so every FMA of every lane is useful work -- on GB300 the
 // FP64 pipe is the bottleneck, and this layout issues no wasted FP64
-// instruction. The triangle is staged once per CTA in packed row-major form
-// (broadcast reads) when it fits, else read through L1 from global memory.
+// instruction. The triangle is staged once per CTA in groups of four rows
+// (tri_group; broadcast reads) when it fits, else read through L1 from global
+// memory.
 //
 // The same kernel serves the variable-size TRSM (kblas{S,D}trsm_vbatch, the
 // reference's non-uniform kblas_trsm_batch overload, MAGMA-only there):
@@ -50,9 +51,18 @@ struct TriDesc {
 __host__ __device__ __forceinline__ size_t tri_x_elems(int vc, int ldx, bool staged) {
   return staged ? ((size_t)vc * ldx + 3) & ~(size_t)3 : (size_t)vc * ldx;
 }
-// The staged triangle: groups of four rows, the four entries of a column side by
-// side (zeros right of the diagonal and below the last row); group g starts here.
-__host__ __device__ __forceinline__ int tri_row4(int g) { return 8 * g * (g + 1); }
+// The staged triangle, without its diagonal: full groups of four rows, group g here;
+// first the columns before 4 g, the four entries of a column side by side, then the
+// six entries within the group row by row and two unused. K - K / 4 * 4 remainder rows
+// follow, each by itself. This is smaller than the packed triangle with its diagonal,
+// so no order keeps fewer vectors or CTAs on an SM than the packed form would (with a
+// 4 x 4 square to a group and full remainder groups, 64 FP64 vectors of order 116 did not
+// leave room for a second CTA: TRSM of 1,500 3939 us, packed 2022).
+__host__ __device__ __forceinline__ int tri_group(int g) { return 8 * g * g; }
+// Remainder row u (0..2) behind G groups.
+__host__ __device__ __forceinline__ int tri_rest(int G, int u) {
+  return tri_group(G) + u * 4 * G + u * (u - 1) / 2;
+}
 
 template <typename T>
 __device__ __forceinline__ void tri_ld4(const T *p, T (&m)[4]) {
@@ -66,6 +76,16 @@ __device__ __forceinline__ void tri_ld4(const T *p, T (&m)[4]) {
 #pragma unroll
     for (int u = 0; u < 4; u++) m[u] = p[u];
   }
+}
+
+template <typename T>
+__device__ __forceinline__ void tri_ld6(const T *p, T (&m)[6]) {
+  T lo[4];
+  tri_ld4(p, lo);
+#pragma unroll
+  for (int u = 0; u < 4; u++) m[u] = lo[u];
+  m[4] = p[4];
+  m[5] = p[5];
 }
 
 // s[u] = sum over k < i0 of M(i0 + u, k) x[k], i0 a multiple of 4, even and odd
@@ -95,7 +115,7 @@ __device__ __forceinline__ void tri_rows4(const T *g, const T *x, int i0, T (&s)
   for (int u = 0; u < 4; u++) s[u] = e[u] + o[u];
 }
 
-// The same sum for one row: the last rows when their number is no multiple of four
+// The same sum for one row g: the last rows when their number is no multiple of four
 // (the FMAs of rows that are not there would cost as much as others: 40% of them at
 // order 9).
 template <typename T>
@@ -104,10 +124,10 @@ __device__ __forceinline__ T tri_row1(const T *g, const T *x, int n) {
   int k = 0;
 #pragma unroll 2
   for (; k + 1 < n; k += 2) {
-    e += g[4 * k] * x[k];
-    o += g[4 * k + 4] * x[k + 1];
+    e += g[k] * x[k];
+    o += g[k + 1] * x[k + 1];
   }
-  if (k < n) e += g[4 * k] * x[k];
+  if (k < n) e += g[k] * x[k];
   return e + o;
 }
 
@@ -163,7 +183,7 @@ __global__ void tri_vec_kernel(TriDesc d, T alpha, AccA A, AccB B, Dims dims, lo
 
   T *sX = reinterpret_cast<T *>(smem_raw);       // VC x ldx
   T *sD = sX + tri_x_elems(d.VC, d.ldx, d.staged);         // K diagonal entries (or reciprocals)
-  T *sM = sD + ((d.Kmax + 3) & ~3);              // staged triangle, see tri_row4
+  T *sM = sD + ((d.Kmax + 3) & ~3);              // staged triangle, see tri_group
   const T *Ag = A.get(mat);
   T *Bg = B.get(mat);
 
@@ -193,9 +213,17 @@ __global__ void tri_vec_kernel(TriDesc d, T alpha, AccA A, AccB B, Dims dims, lo
     sD[i] = (OP == 0) ? T(1) / dg : dg;
   }
   if (d.staged)
-    for (int i = tid; i < ((K + 3) & ~3); i += NT) {
-      T *dst = sM + tri_row4(i >> 2) + (i & 3);
-      for (int k = 0; k < (i | 3); k++) dst[4 * k] = (k < i && i < K) ? Mval(i, k) : T(0);
+    for (int i = tid; i < K; i += NT) {
+      const int g = i >> 2, u = i & 3;
+      if (4 * g + 4 <= K) {
+        T *dst = sM + tri_group(g);
+        for (int k = 0; k < 4 * g; k++) dst[4 * k + u] = Mval(i, k);
+        dst += 16 * g + u * (u - 1) / 2;
+        for (int k = 4 * g; k < i; k++) dst[k - 4 * g] = Mval(i, k);
+      } else {
+        T *dst = sM + tri_rest(g, u);
+        for (int k = 0; k < i; k++) dst[k] = Mval(i, k);
+      }
     }
 
   for (int c = blockIdx.y; c < nchunks; c += gridDim.y) {
@@ -219,35 +247,37 @@ __global__ void tri_vec_kernel(TriDesc d, T alpha, AccA A, AccB B, Dims dims, lo
       } else if (OP == 0) {
         int i0 = 0;
         for (; i0 + 4 <= K; i0 += 4) {
-          T s[4];
-          if (i0 > 0) tri_rows4(sM + tri_row4(i0 >> 2), x, i0, s);
-          const T *tr = sM + tri_row4(i0 >> 2) + 4 * i0;  // (row, i0 + v) at tr[4 v + row - i0]
+          const T *gr = sM + tri_group(i0 >> 2);
+          T s[4], tr[6];  // (i0 + u, i0 + q) in tr[u (u - 1) / 2 + q]
+          if (i0 > 0) tri_rows4(gr, x, i0, s);
+          tri_ld6(gr + 4 * i0, tr);
 #pragma unroll
           for (int u = 0; u < 4; u++) {
             T v = i0 > 0 ? x[i0 + u] - s[u] : x[i0 + u];
 #pragma unroll
-            for (int q = 0; q < u; q++) v -= tr[4 * q + u] * s[q];
+            for (int q = 0; q < u; q++) v -= tr[u * (u - 1) / 2 + q] * s[q];
             s[u] = v * sD[i0 + u];  // solved
             x[i0 + u] = s[u];
           }
         }
         for (int i = i0; i < K; i++)
-          x[i] = (x[i] - tri_row1(sM + tri_row4(i0 >> 2) + (i - i0), x, i)) * sD[i];
+          x[i] = (x[i] - tri_row1(sM + tri_rest(i0 >> 2, i - i0), x, i)) * sD[i];
       } else {
         const int full = K & ~3;
         for (int i = K - 1; i >= full; i--) {
-          const T s = tri_row1(sM + tri_row4(full >> 2) + (i - full), x, i) + sD[i] * x[i];
+          const T s = tri_row1(sM + tri_rest(full >> 2, i - full), x, i) + sD[i] * x[i];
           x[i] = alpha == T(1) ? s : alpha * s;
         }
         for (int i0 = full - 4; i0 >= 0; i0 -= 4) {
-          T s[4], xi[4];
-          tri_rows4(sM + tri_row4(i0 >> 2), x, i0, s);
-          const T *tr = sM + tri_row4(i0 >> 2) + 4 * i0;
+          const T *gr = sM + tri_group(i0 >> 2);
+          T s[4], tr[6], xi[4];
+          tri_rows4(gr, x, i0, s);
+          tri_ld6(gr + 4 * i0, tr);
 #pragma unroll
           for (int u = 0; u < 4; u++) {
             xi[u] = x[i0 + u];
 #pragma unroll
-            for (int q = 0; q < u; q++) s[u] += tr[4 * q + u] * xi[q];
+            for (int q = 0; q < u; q++) s[u] += tr[u * (u - 1) / 2 + q] * xi[q];
             s[u] += sD[i0 + u] * xi[u];
           }
 #pragma unroll
@@ -283,7 +313,7 @@ static int plan_tri(KBlasHandle *h, char side, char uplo, char trans, char diag,
   d.Kmax = Kmax;
   d.ldx = Kmax | 1;
   const int limit = max_smem(h);
-  const size_t tri_bytes = (size_t)tri_row4((Kmax + 3) >> 2) * sizeof(T);
+  const size_t tri_bytes = (size_t)tri_rest(Kmax >> 2, Kmax & 3) * sizeof(T);
   d.staged = (size_t)Kmax * (Kmax + 1) / 2 * sizeof(T) <= 64 * 1024;
   int VC = Vmax < 64 ? Vmax : 64;
   if (VC < 1) VC = 1;
