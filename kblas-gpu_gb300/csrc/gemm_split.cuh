@@ -345,10 +345,13 @@ constexpr int SP_SMEM = SP_SMEM_A + SP_SMEM_B;
 // matrices, FP64-FMA tiles against split: 16^3 325 / 493 us, 24 x 24 x 16
 // 622 / 541, 32 x 32 x 16 622 / 541, 24^3 1148 / 555, 64 x 64 x 16 2450 / 934,
 // 64^3 8771 / 1049; 5,000 of 128 x 16 x 64 2299 / 341, of 128^3 17839 / 1784. A tile
-// costs the split kernel about the same whatever its fill, hence the product;
-// below k = 16 its error is no longer smaller than that of an FP64 chain.
+// costs the split kernel about the same whatever its fill, hence the product; the FP64
+// tiles do half their work for up to 16 rows and k in steps of 16, so there one step
+// stays with them (16 x 48 x 16 637 / 823, 16 x 64 x 16 635 / 851, 8 x 128 x 16 1264 /
+// 1478, but 16 x 48 x 24 1177 / 823). Below k = 16 the error of the split is no longer
+// smaller than that of an FP64 chain.
 static inline bool sp_worthwhile(int m, int n, int k) {
-  return k >= 16 && (long long)m * n * k >= 24 * 24 * 16;
+  return k >= 16 && (k > 16 || m > 16) && (long long)m * n * k >= 24 * 24 * 16;
 }
 
 // Grid of a split launch: row tiles of the largest matrix, each with as many
