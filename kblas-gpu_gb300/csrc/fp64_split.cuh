@@ -10,18 +10,19 @@
 // cuts the operands and puts the results together.
 //
 // Each row of op(A) (and each column of op(B)) gets a power-of-two scale
-// 2^E > |x| and every element becomes a 56-bit fixed-point number
-// round(x 2^(55 - E)) = sum_i s_i 2^(8 (7 - i)), i = 1..7, with signed 8-bit
+// 2^E > |x| and every element becomes a 56-bit fixed-point number,
+// x 2^(55 - E) cut towards zero = sum_i s_i 2^(8 (7 - i)), i = 1..7, with signed 8-bit
 // digits s_i in [-128, 127] held exactly in FP16. The products s_i s_j' with
 // i + j <= 8 are summed on the tensor cores; all with the same i + j share an
 // FP32 accumulator, which stays exact: with at most 4 products per
 // accumulator and a k chunk of 64 it is an integer of at most 2^22. The seven
 // sums are put together in 64-bit integers and rounded once to FP64.
 //
-// Error: the cut loses 2^-56 2^E per element and the dropped products
-// (i + j = 9) at most 6 2^-56 2^(Ei + Ej) per k (about 2^-56 in the mean), so
-// against sum_k |a_ik| |b_kj| the result is as accurate as a chain of FP64
-// FMAs whenever that sum is not far below 2^(Ei + Ej). That is checked for
+// Error: the cut loses up to 2^-55 2^E per element, always towards zero (2^-56 in
+// the mean), and the dropped products (i + j = 9) are at most 6 2^-56 2^(Ei + Ej) per
+// k (about 2^-56 in the mean), so against sum_k |a_ik| |b_kj| the result is as
+// accurate as a chain of FP64 FMAs over 16 k or more whenever that sum is not far
+// below 2^(Ei + Ej); shorter sums use FP64 FMAs. The former is checked for
 // every entry: one more product, of |s_1| with |s_1'|, estimates the sum, and
 // an entry whose estimate is below 2^-2 2^(Ei + Ej) is computed again with
 // FP64 FMAs (graded or sparse data; at most a few entries of a dense tile).
@@ -45,6 +46,7 @@ namespace kgb {
 constexpr int SP_TM = 64;    // rows of a tile
 constexpr int SP_TN = 32;    // columns of a tile
 constexpr int SP_KC = 64;    // k chunk (one scale per row and chunk)
+constexpr int SP_KMIN = 16;  // shortest k chunk that is cut (see the error above)
 constexpr int SP_NT = 256;   // threads per CTA
 constexpr int SP_APL = 9;    // A planes: digits 1..7, |digit 1| twice
 constexpr int SP_BPL = 8;    // B planes: digits 1..7, |digit 1|

@@ -81,6 +81,14 @@ __device__ __forceinline__ uint32_t sp_rowmax(uint32_t mx) {
   return mx;
 }
 
+// End of the k chunk that starts at k0. No chunk is shorter than SP_KMIN unless k
+// itself is (a variable-size batch: those use FP64 FMAs): a remainder of 1..15 takes 16
+// of the 64 before it, which costs the same MMAs.
+__device__ __forceinline__ int sp_chunk_end(int k0, int k) {
+  const int left = k - k0;
+  return left <= SP_KC ? k : k0 + (left < SP_KC + SP_KMIN ? SP_KC - SP_KMIN : SP_KC);
+}
+
 // One 64-row tile at I0 against the column tiles cp, cp + ncp, ... (alpha != 0
 // and k > 0). A warp cuts 4 rows at a time, lane = (row, k group): the lanes
 // of a row find its scale by shuffles, and both operand orders load whole
@@ -104,12 +112,13 @@ static __device__ bool sp_row_tile(const SpTile &j, int I0, int cp, int ncp, dou
     if (cp < skip) cp += (skip - cp + ncp - 1) / ncp * ncp;
   }
   if (cp >= tn) return true;
-  for (int k0 = 0; k0 < j.k; k0 += SP_KC) {
-    const int kend = min(j.k, k0 + SP_KC), ksteps = (kend - k0 + 15) >> 4;
+  for (int k0 = 0, kend; k0 < j.k; k0 = kend) {
+    kend = sp_chunk_end(k0, j.k);
+    const int ksteps = (kend - k0 + 15) >> 4;
     const double beta = k0 == 0 ? beta0 : 1.0;
     const bool kon = 8 * kg < 16 * ksteps;
     const int kk = k0 + 8 * kg;
-    int special = 0;
+    int special = kend - k0 < SP_KMIN;
     double xb[8];
     {
       double x0[8], x1[8];
@@ -117,7 +126,7 @@ static __device__ bool sp_row_tile(const SpTile &j, int I0, int cp, int ncp, dou
       sp_load8(j.A, I0 + rsub + 32, rsub + 32 < rows, kk, kend, x1);
       sp_load8(j.B, cp * SP_TN + rsub, cp * SP_TN + rsub < j.n, kk, kend, xb);
       const uint32_t m0 = sp_rowmax(sp_maxbits(x0)), m1 = sp_rowmax(sp_maxbits(x1));
-      special = sp_special(m0) || sp_special(m1);
+      special |= sp_special(m0) || sp_special(m1);
       const int e0 = sp_scale(m0), e1 = sp_scale(m1);
       if (kg == 0) {
         s.eA[rsub] = e0;
