@@ -200,6 +200,10 @@ static inline int plan_redo(KBlasHandle *h, int max_n, PosvPlan &pl) {
   return st;
 }
 
+// Uniform plain FP64 batches run in slices of this many systems, so that the list of
+// those left to the FP64 path has a fixed size (256 KB).
+constexpr long long FIX_SLICE = 65536;
+
 // Device workspace layout shared by the uniform mixed and the variable-size
 // routines (offsets in bytes from the start of the handle's device data).
 struct PosvWs {
@@ -209,14 +213,15 @@ struct PosvWs {
   size_t off = 0;      // int[max_n + 1]   first slot of order n in perm
   size_t ioff = 0;     // int[max_n + 1]   first item of order n
   size_t cursor = 0;   // int[max_n + 1]
-  size_t redo = 0;     // int[batch]        plain FP64: systems for the FP64 path
+  size_t redo = 0;     // int[batch], uniform int[FIX_SLICE]: plain FP64: systems for the FP64 path
   size_t perm = 0;     // int[batch]
   size_t items = 0;    // int4[batch]
   size_t scratch = 0;  // grid * slot_bytes
   size_t total = 0;
 };
 
-// fix: the plain FP64 routines, whose systems run in fixed point first.
+// fix: the plain FP64 routines, whose systems run in fixed point first. The uniform
+// layouts do not depend on the batch: a workspace queried for one batch serves any.
 static inline PosvWs posv_ws_layout(KBlasHandle *h, int max_n, long long batch, bool binned,
                                     bool fix, const PosvPlan &pl) {
   PosvWs w;
@@ -234,7 +239,7 @@ static inline PosvWs posv_ws_layout(KBlasHandle *h, int max_n, long long batch, 
     w.ioff = take(nb);
     w.cursor = take(nb);
   }
-  if (fix) w.redo = take((size_t)batch * sizeof(int));
+  if (fix) w.redo = take((size_t)(binned ? batch : FIX_SLICE) * sizeof(int));
   if (binned) {
     w.perm = take((size_t)batch * sizeof(int));
     w.items = take((size_t)batch * sizeof(int4));

@@ -1,5 +1,5 @@
 // posv_vbatch.cu -- variable-size batched DPOSV (plain FP64 and mixed
-// precision) in one persistent launch, preceded by on-device binning.
+// precision) in persistent launches, preceded by on-device binning.
 //
 // KBLAS has no variable-size POTRF/POSV (its non-uniform TRSM/SYRK forward to
 // MAGMA, src/batch_triangular/Xtrsm_batch_drivers.cuh:278); the argument
@@ -149,11 +149,12 @@ size_t vbatch_ws_bytes(KBlasHandle *h, int max_n, long long batch, bool mixed) {
   return posv_ws_layout(h, max_n, batch, true, !mixed && max_n > 32, panel).total;
 }
 
-// Uniform FP64 POSV / POTRF / POTRS (op 0 / 1 / 2) of order n > 32 on the
-// persistent panel path: one launch, teams sized by the FP64 tuning table.
-// Returns KBLAS_InsufficientWorkspace, launching nothing, when the handle's
-// workspace is short of fp64_uniform_ws_bytes (the caller then uses the
-// one-launch blocked kernel); arguments are checked by the caller.
+// Uniform FP64 POSV / POTRF / POTRS (op 0 / 1 / 2) of order n > 32 in fixed point and,
+// what that leaves, on the FP64 panel path with teams sized by the tuning table: a
+// memset and two launches per FIX_SLICE systems (POTRS: one). Returns
+// KBLAS_InsufficientWorkspace, launching nothing, when the handle's workspace is short
+// of fp64_uniform_ws_bytes (the caller then uses the one-launch blocked kernel);
+// arguments are checked by the caller.
 size_t fp64_uniform_ws_bytes(KBlasHandle *h, int n, long long batch) {
   if (n <= 32 || n > PC_MAX_N || batch <= 0) return 0;
   PosvPlan pl;
@@ -171,19 +172,13 @@ int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, i
   if (ws.total > h->ws.allocated.d_data_bytes || !h->ws.d_data) return KBLAS_InsufficientWorkspace;
   char *base = static_cast<char *>(h->ws.d_data);
   int *header = reinterpret_cast<int *>(base + ws.header);
-  cudaError_t e = cudaMemsetAsync(header, 0, 64 * sizeof(int), h->stream);
-  if (e != cudaSuccess) return cuda_check(e, "cudaMemsetAsync", __FILE__, __LINE__);
   sys.n = n;
   sys.m = (op == 1) ? 0 : m;
   sys.op = (op == 2) ? 2 : 0;
   FixArgs fa{};
-  fa.info = info;
   fa.redo_count = header + 1;
   fa.redo_list = reinterpret_cast<int *>(base + ws.redo);
   fa.scratch = reinterpret_cast<double *>(base + ws.scratch);
-  st = fix_launch(h, n, batch, sys, fa, header + 16);
-  if (st != KBLAS_Success || op == 2) return st;
-  // what the fixed-point kernel left: FP64
   ItemArgs it{};
   it.uniform = 2;
   it.n_uniform = n;
@@ -192,10 +187,29 @@ int fp64_uniform_persistent(KBlasHandle *h, int op, int m, int n, SysArgs sys, i
   it.queue = header;
   it.few_max = PC_FEW;
   it.few = few_cfg();
-  OutArgs out{info, nullptr, base + ws.scratch, (long long)pl.slot_bytes,
-              0, h->d_status};
-  posv_persistent_kernel<false, 2><<<pl.grid, PC_NT, pl.smem, h->stream>>>(sys, it, out, pl.cfg, pl.smem);
-  KGB_LAUNCH_CHECK("posv_persistent_kernel<fp64>");
+  for (long long first = 0; first < batch; first += FIX_SLICE) {
+    const long long count = batch - first < FIX_SLICE ? batch - first : FIX_SLICE;
+    SysArgs part = sys;
+    if (sys.mode == 0) {
+      part.A += first * sys.sA;
+      if (part.B) part.B += first * sys.sB;
+    } else {
+      part.Aarr += first;
+      if (part.Barr) part.Barr += first;
+    }
+    int *const info_part = info ? info + first : nullptr;
+    cudaError_t e = cudaMemsetAsync(header, 0, 64 * sizeof(int), h->stream);
+    if (e != cudaSuccess) return cuda_check(e, "cudaMemsetAsync", __FILE__, __LINE__);
+    fa.info = info_part;
+    st = fix_launch(h, n, count, part, fa, header + 16);
+    if (st != KBLAS_Success) return st;
+    if (op == 2) continue;
+    // what the fixed-point kernel left: FP64
+    OutArgs out{info_part, nullptr, base + ws.scratch, (long long)pl.slot_bytes,
+                0, h->d_status};
+    posv_persistent_kernel<false, 2><<<pl.grid, PC_NT, pl.smem, h->stream>>>(part, it, out, pl.cfg, pl.smem);
+    KGB_LAUNCH_CHECK("posv_persistent_kernel<fp64>");
+  }
   return KBLAS_Success;
 }
 
