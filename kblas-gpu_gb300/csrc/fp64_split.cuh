@@ -154,8 +154,7 @@ __host__ __device__ __forceinline__ uint32_t idesc_f16_f32(int M, int N) {
 // thread. TMEM columns 32 c .. 32 c + 31, c = 0..6: lanes 0..63 hold the sum
 // of the products with i + j = c + 2, lanes 64..127 those with i + j = c + 3
 // (c <= 5); c = 7: the estimate, in both halves.
-__device__ __forceinline__ void sp_issue(uint32_t tmem, uint32_t sA, uint32_t sB, int ksteps,
-                                         bool estimate) {
+__device__ __forceinline__ void sp_issue(uint32_t tmem, uint32_t sA, uint32_t sB, int ksteps) {
   for (int ks = 0; ks < ksteps; ks++) {
     const uint32_t a = sA + (uint32_t)ks * 2 * SP_LBO_A, b = sB + (uint32_t)ks * 2 * SP_LBO_B;
     const uint64_t bd = smem_desc(b, SP_LBO_B, SP_SBO);
@@ -165,10 +164,9 @@ __device__ __forceinline__ void sp_issue(uint32_t tmem, uint32_t sA, uint32_t sB
       tc_mma_bf16(tmem + 64 * p, ad, bd, idesc_f16_f32(128, SP_TN * (7 - 2 * p)),
                   (ks | p) ? 1u : 0u);
     }
-    if (estimate)
-      tc_mma_bf16(tmem + 224, smem_desc(a + 7 * SP_TM * 16, SP_LBO_A, SP_SBO),
-                  smem_desc(b + 7 * SP_TN * 16, SP_LBO_B, SP_SBO), idesc_f16_f32(128, SP_TN),
-                  ks ? 1u : 0u);
+    tc_mma_bf16(tmem + 224, smem_desc(a + 7 * SP_TM * 16, SP_LBO_A, SP_SBO),
+                smem_desc(b + 7 * SP_TN * 16, SP_LBO_B, SP_SBO), idesc_f16_f32(128, SP_TN),
+                ks ? 1u : 0u);
   }
 }
 

@@ -151,7 +151,7 @@ static __device__ bool sp_row_tile(const SpTile &j, int I0, int cp, int ncp, dou
       const bool native = __syncthreads_or(special) != 0;
       if (!native && tid == 0) {
         tc_fence_after_sync();
-        sp_issue(s.tmem, smem_addr(sA), smem_addr(sB), ksteps, true);
+        sp_issue(s.tmem, smem_addr(sA), smem_addr(sB), ksteps);
         tc_commit(&s.bar);
       }
       const int gi = I0 + row, c0 = 16 * half + (lower ? 8 : 0);  // the 8 columns this thread finishes
