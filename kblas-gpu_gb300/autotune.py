@@ -7,6 +7,8 @@ CTA, one system per team, so the useful item size is the number of teams
 (256 / team size); the choice that matters is the team size. For each class
 this sweeps every team size the kernels accept, times the variable-size POSV
 on a batch whose orders are log-uniform over that class, and keeps the fastest.
+The plain FP64 launch of the classes above n = 32 takes what the fixed-point
+kernels leave, so there every matrix is scaled by 2^850, beyond their range.
 The chosen table is applied at run time through kblasSetPosvTuning while it
 is measured, and written out as a header to be compiled in.
 
@@ -101,9 +103,17 @@ class ClassBatch:
         self.info = torch.zeros(batch, dtype=torch.int32, device="cuda")
         self.iter = torch.zeros(batch, dtype=torch.int32, device="cuda")
         self.max_n = int(ns.max())
+        self.A0_form = self.A0
+
+    def scale(self, form, c):
+        """The matrices that the launch shaped by class c of this form takes."""
+        if form == "plain" and NMAX[c] > 32:
+            self.A0_form = self.A0 * 2.0 ** 850
+        else:
+            self.A0_form = self.A0
 
     def restore(self):
-        self.A.copy_(self.A0)
+        self.A.copy_(self.A0_form)
         self.B.copy_(self.B0)
 
 
@@ -223,6 +233,7 @@ def tune(torch, kb, reps=5, log=print):
             ms_table = {}
             for c in range(NCLS):
                 cb = batches[c]
+                cb.scale(form, c)
                 res = {}
                 for ts in CANDIDATES[c]:
                     trial_ts, trial_spi = list(best_ts), list(best_spi)
@@ -237,6 +248,7 @@ def tune(torch, kb, reps=5, log=print):
                 ts = min(res, key=res.get)
                 best_ts[c], best_spi[c] = ts, NT // ts
                 ms_table[c] = res
+                cb.A0_form = cb.A0
             out[form] = {"ts": best_ts, "spi": best_spi, "ms": ms_table}
     finally:
         kb.lib().kblasSetPosvTuning(1, None, None, None)
