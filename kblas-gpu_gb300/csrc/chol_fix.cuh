@@ -22,21 +22,27 @@
 // So an entry far below sqrt(a_ii a_jj) would keep fewer bits than in FP64, and a
 // component of a solution that hangs on such entries alone (the far end of a
 // decaying covariance for a unit right-hand side, weakly coupled unknowns) would
-// be wrong in as many. So these are counted (fx_weak): a coupling of the unknowns
+// be wrong in as many. So these are counted (fx_share): a coupling of the unknowns
 // i > j is an entry with a_ij or S(i, j) not zero, t the bits by which the larger of
 // both lies below its scale 2^(E_i + E_j), and an unknown whose couplings have
 // max(0, t - 8) at more than 1 in the mean leaves the matrix to the FP64 path.
-// (Single small entries among others of the same unknowns, as random matrices have
+// Single small entries among others of the same unknowns, as random matrices have
 // them, do not matter: the others' rounding reaches every component that theirs
-// reaches.) Against quad precision, FP64 FMAs / fixed point, on the matrices that
-// stay: root mean square of |A - L L^T|_ij / (|L| |L^T|)_ij in 2^-53, G G^T + n I of
-// order 128 1.2 / 1.0, condition 1e6 of order 64 0.5 / 0.4, squared-exponential
-// covariance of length 0.3 and order 160 0.35 / 0.41; the largest relative error of a
-// component of A^-1 e_1 7e-14 / 4e-13, 4e-10 / 5e-11 and 1.8e-9 / 1.5e-9. The same
-// covariance with length 0.05, taken in fixed point: 3e-11 / 3e-6. 56-bit entries with
-// the cross products summed in FP32 are faster (10,000 POSV of order 64, four right-hand
-// sides 968 us against 1139, 2,000 of order 150 1944 against 2405), but not as accurate
-// as FP64 FMAs entry by entry: 1.2 / 4.8 on the shifted matrices.
+// reaches. That takes others that lead there: a matrix that has a coupling with t
+// above 12 stays only if every unknown has couplings with t up to 12 to at least half
+// of the unknowns, for then the two that it couples have at least two such neighbours
+// in common. (Two strongly coupled halves of order 110 with one coupling of 1e-12
+// between them, taken in fixed point: the components of A^-1 e_1 in the second half
+// wrong by 2e-6.)
+// Against quad precision, FP64 FMAs / fixed point, on the matrices that stay: root mean
+// square of |A - L L^T|_ij / (|L| |L^T|)_ij in 2^-53, G G^T + n I of order 128 1.2 /
+// 1.0, condition 1e6 of order 64 0.5 / 0.4, squared-exponential covariance of length
+// 0.3 and order 160 0.35 / 0.41; the largest relative error of a component of A^-1 e_1
+// 7e-14 / 4e-13, 4e-10 / 5e-11 and 1.8e-9 / 1.5e-9. The same covariance with length
+// 0.05, taken in fixed point: 3e-11 / 3e-6. 56-bit entries with the cross products
+// summed in FP32 are faster (10,000 POSV of order 64, four right-hand sides 968 us
+// against 1139, 2,000 of order 150 1944 against 2405), but not as accurate as FP64 FMAs
+// entry by entry: 1.2 / 4.8 on the shifted matrices.
 //
 // A matrix that does not fit the scheme -- a pivot below 2^-42 a_jj, an entry
 // or a row of L above its bound (only when A is not positive definite), an
@@ -208,17 +214,39 @@ __device__ __forceinline__ void fx_ld8(const double *p, double (&y)[FX_W]) {
     y[c + 1] = v.y;
   }
 }
-// A coupling's share of its two unknowns' sums, plus 1 (so 1 if there is none): an
-// unknown whose sum of shares ends above zero has couplings that are too weak. Where the line lies: an
-// entry's error is about 2^-59..2^-60 of its scale, which FP64 FMAs reach 6 bits below
-// it, and with 8 bits free and 1 more in the mean all of G G^T + n I up to order 1024
-// (0.0..0.5 in the mean of the worst unknown) and random matrices of condition
-// 1e2..1e8 (0.0..0.2) stay; squared-exponential covariances on the unit square stay
-// from length 0.27 on (at 0.25 1.3..2.2, at 0.2 2.3..5.8).
-__device__ __forceinline__ int fx_weak(long long a, long long s) {
+// The bits by which a coupling lies below its scale, plus 2; 32: it has none of the upper
+// 30 or is none at all.
+__device__ __forceinline__ int fx_below(long long a, long long s) {
   const int ah = (int)(a >> 32), sh = (int)(s >> 32);
-  const int z = __clz((ah ^ (ah >> 31)) | (sh ^ (sh >> 31)));  // 2 at the scale
-  return (a | s) == 0 ? 1 : max(z - 10, 0);
+  return __clz((ah ^ (ah >> 31)) | (sh ^ (sh >> 31)));
+}
+// A coupling's share of its two unknowns' sums: an unknown whose sum of shares ends above
+// zero has couplings that are too weak. Where the line lies: an entry's error is about
+// 2^-59..2^-60 of its scale, which FP64 FMAs reach 6 bits below it, and with 8 bits free
+// and 1 more in the mean all of G G^T + n I up to order 1024 (0.0..0.5 in the mean of the
+// worst unknown) and random matrices of condition 1e2..1e8 (0.0..0.2) stay;
+// squared-exponential covariances on the unit square stay from length 0.27 on (at 0.25
+// 1.3..2.2, at 0.2 2.3..5.8).
+__device__ __forceinline__ int fx_share(bool none, int below) {
+  return none ? 0 : max(below - 10, 0) - 1;
+}
+// Couplings more than 12 bits below their scales (an entry that is the only way from one
+// unknown to another is then good to 2^-47) and pairs without a coupling: rare in dense
+// matrices, so these are not summed like the shares but added at once, to the upper half
+// of both unknowns' sums. weak gets bit 0 if it is a coupling.
+constexpr int FX_LOOSE = 14;  // of fx_below
+constexpr int FX_COUNT = 1 << 16;
+__device__ __forceinline__ void fx_count_loose(bool none, int *wi, int *wj, unsigned &weak) {
+  if (!none) weak |= 1u;
+  atomicAdd(wi, FX_COUNT);
+  atomicAdd(wj, FX_COUNT);
+}
+// Whether an unknown's sum leaves the matrix to FP64; weak gets bit 1 if the unknown is
+// strongly coupled to fewer than half of the unknowns.
+__device__ __forceinline__ bool fx_too_weak(int sum, int n, unsigned &weak) {
+  const int shares = (short)sum, loose = (sum - shares) / FX_COUNT;
+  if (2 * (n - 1 - loose) < n) weak |= 2u;
+  return shares > 0;
 }
 
 // R rows of a thread against the block of columns C..C+7: the sums over the
@@ -355,7 +383,7 @@ __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C
                                            long long (&hh)[R][FX_W], long long (&mid)[R][FX_W],
                                            long long (&a)[R][FX_W], FixScratch *fs,
                                            float (&qs)[R], int *wk, int (&wr)[R],
-                                           unsigned &bad)
+                                           unsigned &weak, unsigned &bad)
 {
   const int lane = threadIdx.x & 31;
   const int ld = F.ld(C / FX_W);
@@ -391,9 +419,11 @@ __device__ __forceinline__ bool fx_columns(const FixLayout &F, double *Xs, int C
           const float f = (float)__double2hiint(x[r]);
           qs[r] += f * f;
           if (row[r] > C + c) {
-            const int w = fx_weak(a[r][c], s[r]) - 1;
+            const bool none = (a[r][c] | s[r]) == 0;
+            const int below = fx_below(a[r][c], s[r]), w = fx_share(none, below);
             wr[r] += w;
             wc[c >> 2] += (unsigned)w << (8 * (c & 3));
+            if (below > FX_LOOSE) fx_count_loose(none, wk + row[r], wk + C + c, weak);
           }
         }
       }
@@ -427,7 +457,7 @@ __device__ __forceinline__ bool fx_rows(const FixLayout &F, const double *A, int
                                         int C, const int (&row)[R], const bool (&own)[R],
                                         const int *Es, float *q, int *wk, int *zs,
                                         double *rho_s, FixScratch *fs, FixStage *st,
-                                        unsigned &bad)
+                                        unsigned &weak, unsigned &bad)
 {
   int ri[R];
   long long a[R][FX_W], hh[R][FX_W], mid[R][FX_W];
@@ -461,7 +491,7 @@ __device__ __forceinline__ bool fx_rows(const FixLayout &F, const double *A, int
 #pragma unroll
   for (int r = 0; r < R; r++) qs[r] = 0.f, wr[r] = 0;
   const bool ok =
-      fx_columns<R, FIRST, BIG>(F, Xs, C, row, own, zs, rho_s, hh, mid, a, fs, qs, wk, wr, bad);
+      fx_columns<R, FIRST, BIG>(F, Xs, C, row, own, zs, rho_s, hh, mid, a, fs, qs, wk, wr, weak, bad);
   // a row whose squares add up to more than a_ii: A is not positive definite
 #pragma unroll
   for (int r = 0; r < R; r++)
@@ -481,7 +511,7 @@ template <int NW, int R, bool BIG>
 __device__ __forceinline__ bool fx_block(const FixLayout &F, const double *A, int lda, double *Xs,
                                          int C, const int *Es, float *q, int *wk, int *zs,
                                          double *rho_s, FixScratch *fs, FixStage *st,
-                                         unsigned &bad)
+                                         unsigned &weak, unsigned &bad)
 {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int row[R];
@@ -496,7 +526,7 @@ __device__ __forceinline__ bool fx_block(const FixLayout &F, const double *A, in
   // the pivots at the barrier
   bool ok = true;
   if (w == 0 || C + w * (32 - FX_W) + FX_W < F.n)
-    ok = fx_rows<R, true, BIG>(F, A, lda, Xs, C, row, own, Es, q, wk, zs, rho_s, fs, st, bad);
+    ok = fx_rows<R, true, BIG>(F, A, lda, Xs, C, row, own, Es, q, wk, zs, rho_s, fs, st, weak, bad);
   if (BIG && R == 2) {
     for (int g = C + FX_W + NW * (64 - FX_W); ok && g < F.n; g += NW * 64) {
 #pragma unroll
@@ -504,14 +534,14 @@ __device__ __forceinline__ bool fx_block(const FixLayout &F, const double *A, in
         row[r] = g + (w * R + r) * 32 + lane;
         own[r] = row[r] < F.n;
       }
-      fx_rows<R, false, BIG>(F, A, lda, Xs, C, row, own, Es, q, wk, zs, rho_s, fs, st, bad);
+      fx_rows<R, false, BIG>(F, A, lda, Xs, C, row, own, Es, q, wk, zs, rho_s, fs, st, weak, bad);
     }
   }
   if (NW == 1) __syncwarp();
   else ok = __syncthreads_and(ok);
   // the sums of this block's unknowns are complete and stay as they are
   const int i = C + (lane & (FX_W - 1));
-  return ok && !__any_sync(0xffffffffu, i < F.n && wk[i] > 0);
+  return ok && !__any_sync(0xffffffffu, i < F.n && fx_too_weak(wk[i], F.n, weak));
 }
 
 // Cholesky factor of the lower triangle of A into Xs (limbs), by a CTA of NW
@@ -533,15 +563,16 @@ __device__ __forceinline__ bool fx_potrf(const FixLayout &F, const double *A, in
   else b = __syncthreads_or(b);
   if (b) return false;
   if (NW == 1) __syncwarp();
-  unsigned bad = 0;
+  unsigned bad = 0, weak = 0;
   bool ok = true;
   int C = 0;
   if (RMAX > 1)
     for (; ok && F.n - C > FX_W + NW * (32 - FX_W); C += FX_W)
-      ok = fx_block<NW, 2, BIG>(F, A, lda, Xs, C, Es, q, wk, zs, rho_s, fs, st, bad);
+      ok = fx_block<NW, 2, BIG>(F, A, lda, Xs, C, Es, q, wk, zs, rho_s, fs, st, weak, bad);
   for (; ok && C < F.n; C += FX_W)
-    ok = fx_block<NW, 1, BIG>(F, A, lda, Xs, C, Es, q, wk, zs, rho_s, fs, st, bad);
-  // (ok is the same in every warp)
+    ok = fx_block<NW, 1, BIG>(F, A, lda, Xs, C, Es, q, wk, zs, rho_s, fs, st, weak, bad);
+  // (ok is the same in every warp; each finds every unknown's sum, hence bit 1 of weak)
+  if (__any_sync(0xffffffffu, weak & 2u) && (weak & 1u)) bad = 1;
   if (NW == 1) return ok && !__any_sync(0xffffffffu, bad != 0);
   return !__syncthreads_or(!ok || bad != 0);
 }
