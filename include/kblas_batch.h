@@ -46,7 +46,7 @@ typedef struct KBlasHandle *kblasHandle_t;
  * request scratch for the fixed-point kernels and the FP64 panel kernel behind
  * them and run on these once the workspace is allocated; without it they run
  * on a one-launch blocked kernel that needs none but is many times slower
- * (about 14% of the FP64 peak at n = 64 against 110% with the workspace). Call
+ * (about 14% of the FP64 peak at n = 64 against 93% with the workspace). Call
  * the query and kblasAllocateWorkspace, as KBLAS callers do, before timing
  * these routines.
  * ------------------------------------------------------------------------- */

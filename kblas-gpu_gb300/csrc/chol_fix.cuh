@@ -290,7 +290,7 @@ __device__ __forceinline__ void fx_dot(const FixLayout &F, const double *Xs, int
 // The same with X in global memory: the next 8 columns of the warp's rows and of
 // the pivot rows are copied to shared memory while the current 8 are multiplied,
 // so the latency of L2 is paid once per block, not once per 4 columns (500 systems
-// of order 512: 13.6 -> 11.6 ms). A's 8 columns come last, the same way, and into av
+// of order 512, with 56-bit entries: 13.6 -> 11.6 ms). A's 8 columns come last, the same way, and into av
 // (zeros right of the diagonal and of the matrix): registers that hold them during the
 // products spill.
 struct FixStage {

@@ -31,18 +31,18 @@ __host__ __device__ __forceinline__ size_t fix_smem_bytes(int n) {
 }
 
 // CTAs per SM that the registers are cut for: of one warp twelve (168 registers;
-// with eight, 255 registers, POSV of order 64 took 15% longer), of two warps five
-// (with four, 28% longer at order 80) or, with the factor in L2, the number that
-// the scratch is for: 8 warps to an SM (with 12, 168 registers, 25% longer at
-// order 200).
+// with eight, 255 registers, POSV of order 64 took 16% longer), of two warps five
+// (with four, 17% longer at order 80, 5% shorter at 100) or, with the factor in L2, the
+// number that the scratch is for: 8 warps to an SM (12 would leave 168 registers, fewer
+// than two rows a lane take).
 template <int NW, bool FAC_SMEM>
 __host__ __device__ constexpr int fix_min_ctas() {
   return FAC_SMEM ? (NW == 1 ? 12 : NW == 2 ? 5 : 1) : 8 / NW;
 }
 
 // The solves as a function of their own: inlined, they and the factorization take
-// registers from each other (20,000 of order 64, factor only: 1245 us without spills,
-// up to 1740 with). L and the reciprocals lie at these offsets of the dynamic shared memory.
+// registers from each other (20,000 of order 64, factor only, with 56-bit entries: 1245
+// us without spills, up to 1740 with). L and the reciprocals lie at these offsets of the dynamic shared memory.
 template <int NW>
 __device__ __noinline__ void fix_solve_smem(int n, int rinv_at, double *B, int ldb, int m)
 {

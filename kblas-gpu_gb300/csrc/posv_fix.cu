@@ -14,16 +14,17 @@ namespace kgb {
 // eight systems of one warp to an SM (no barriers, and every warp busy to the last
 // column) until the systems of an SM no longer fit into its share of L2 and a
 // batch has fewer of them than warps: then four of two warps. us (POSV, one
-// right-hand side) for 2 warps in shared memory / 1 / 2 / 4 warps in L2: 6,000 of
-// order 100 1637 / 1745 / 2580 / 2687; 2,000 of 200 - / 2532 / 3481 / 3819; 1,500 of 256
-// - / 3777 / 4419 / 4761; 500 of 400 (4 right-hand sides) - / 5656 / 5078 / 5540.
+// right-hand side) for 2 warps in shared memory / 1 / 2 warps in L2: 6,000 of order 80
+// 1273 / 1483 / -; of 100 2366 / 2352 / -; 2,000 of 200 - / 3752 / 4708; 1,500 of 256
+// - / 5757 / 6309; 500 of 400 (4 right-hand sides) - / 8349 / 7267.
 struct FixClass {
   int lo, hi;
 };
 static const FixClass FIX_CLASSES[FIX_NCLS] = {{32, 64}, {64, 104}, {104, 320}, {320, PC_MAX_N}};
 // A batch of at most two systems per SM waits for single systems: above order 104
 // they get eight warps, the factor in shared memory up to 216 (197 KB). 50 of order
-// 200 1011 -> 358 us, of 400 2811 -> 2047 (two right-hand sides).
+// 200 (two right-hand sides) with one warp each 1402 us, with eight 468; of 400 7450 and
+// 2559.
 static const FixClass FIX_FEW[FIX_NCLS] = {{32, 64}, {64, 104}, {104, 216}, {216, PC_MAX_N}};
 
 template <int NW, bool FAC_SMEM>

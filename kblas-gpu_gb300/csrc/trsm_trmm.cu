@@ -93,7 +93,7 @@ __device__ __forceinline__ void tri_ld6(const T *p, T (&m)[6]) {
 // four FP64 FMAs keep the pipe busy for 256 cycles, so nothing else of a row
 // costs time but the one addition that joins its two sums. Against a row at a
 // time with four partial sums (20,000 triangles of order 64 on 64 vectors, copies
-// of the operands included): TRSM 6450 -> 5666 us, TRMM 6665 -> 5744 us; the FP64
+// of the operands included): TRSM 6450 -> 5693 us, TRMM 6665 -> 5680 us; the FP64
 // pipe needs 4570.
 template <typename T>
 __device__ __forceinline__ void tri_rows4(const T *g, const T *x, int i0, T (&s)[4]) {
